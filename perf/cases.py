@@ -40,28 +40,28 @@ def _case(name, model, batch, prompt, new, *, dtype="bfloat16", ragged=False, po
 def listed():
     return [
         # a short chat turn on the smallest model: a few hundred small launches a token, nothing else
-        _case("chat turn, 0.5B", "qwen2.5-0.5b", 1, 40, 24),
+        _case("chat turn 0.5B", "qwen2.5-0.5b", 1, 40, 24),
         # a chat turn with some history on the usual model: every token reads all weights once
-        _case("chat turn, 7B", "qwen2.5-7b", 1, 300, 24),
+        _case("chat turn 7B", "qwen2.5-7b", 1, 300, 24),
         # a small service: eight requests of unequal length, prompts of a page or two of text
-        _case("eight requests, 7B", "qwen2.5-7b", 8, 1200, 32, ragged=True),
+        _case("eight requests 7B", "qwen2.5-7b", 8, 1200, 32, ragged=True),
         # a full batch of short unequal requests
-        _case("full batch, 7B", "qwen2.5-7b", 64, 320, 12, ragged=True),
+        _case("full batch 7B", "qwen2.5-7b", 64, 320, 12, ragged=True),
         # a document read in portions, so that other work gets in between, then a short answer
-        _case("document in portions, 7B", "qwen2.5-7b", 1, 6000, 6, portion=2048),
+        _case("document in portions 7B", "qwen2.5-7b", 1, 6000, 6, portion=2048),
         # the true 32-bit path: greedy generation, then every position's logits
-        _case("generate and score, 0.5B float32", "qwen2.5-0.5b", 2, 150, 16, dtype="float32", generate=True),
+        _case("generate and score 0.5B float32", "qwen2.5-0.5b", 2, 150, 16, dtype="float32", generate=True),
         # a long prompt on the decoders with recurrent states: the chain of states is the prompt's time
-        _case("long prompt, Zodosun", "zodosun-2k", 1, 3000, 24),
-        _case("long prompt, Rirudra", "rirudra-2k", 1, 3000, 24),
+        _case("long prompt Zodosun", "zodosun-2k", 1, 3000, 24),
+        _case("long prompt Rirudra", "rirudra-2k", 1, 3000, 24),
         # many unequal requests on the same: states and pages of many sequences
-        _case("thirty-two requests, Zodosun", "zodosun-2k", 32, 300, 24, ragged=True),
+        _case("thirty-two requests Zodosun", "zodosun-2k", 32, 300, 24, ragged=True),
         # a full batch whose prompts come in odd portions
-        _case("full batch in portions, Rirudra", "rirudra-2k", 64, 210, 24, ragged=True, portion=77),
+        _case("full batch in portions Rirudra", "rirudra-2k", 64, 210, 24, ragged=True, portion=77),
         # the 32-bit path of a decoder with states
-        _case("four requests, Rirudra float32", "rirudra-2k", 4, 250, 16, dtype="float32", ragged=True),
+        _case("four requests Rirudra float32", "rirudra-2k", 4, 250, 16, dtype="float32", ragged=True),
         # routed experts and windows, an ordinary batch
-        _case("sixteen requests, Pavisun", "pavisun-2k", 16, 500, 24, ragged=True),
+        _case("sixteen requests Pavisun", "pavisun-2k", 16, 500, 24, ragged=True),
     ]
 
 
