@@ -14,8 +14,11 @@
     library matrix product (cuBLAS through torch.mm with float32 output), as
     the reference engine does for all its products
     (src/models/turbo_generic.rs:68-91 -> candle -> cuBLAS);
-  * everything else (the float32 path, mixed operands): the tiled float32
-    FMA kernel of csrc/gemm.cu — never a reduced-precision mode.
+  * float32 operands and result (the float32 path): the FMA kernels of
+    csrc/gemm_f32.cu with the same epilogues, for up to 8 rows and for more;
+  * everything else (mixed operands, rows that are not 16-byte aligned): the
+    row kernel and the tiled FMA kernel of csrc/gemm.cu.  Never a
+    reduced-precision mode.
 """
 from __future__ import annotations
 
@@ -66,6 +69,7 @@ class PendingNorm:
 FUSE_NORM = {"1": True, "0": False}.get(os.environ.get("TQ_FUSE_NORM", ""), "auto")
 FUSED_NORM_MAX_ROWS = 16
 ROW_KERNEL_MAX_ROWS = 16
+F32_ROW_KERNEL_MAX_ROWS = 8
 SKINNY_MAX_ROWS = 64
 # Weights from which a decode product of up to 16 rows runs on the tcgen05 kernel (see _tc_takes)
 TC_DECODE_MIN_WEIGHT_BYTES = 24 << 20      # the product after a pending norm
@@ -222,6 +226,24 @@ def gemv_rows(x, w, out, bias=None, accumulate=False, swiglu=False, activation=e
     return out
 
 
+def _f32_ok(x, w, out) -> bool:
+    """What csrc/gemm_f32.cu takes: float32 throughout, 16-byte pieces along K, rows that do not overlap."""
+    K = x.shape[1]
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32 and K % 4 == 0
+            and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+            and (x.shape[0] == 1 or (x.stride(0) >= K and out.stride(0) >= out.shape[1])) and w.stride(0) >= K)
+
+
+def gemm_f32(x, w, out, bias=None, accumulate=False, swiglu=False, activation=elementwise.ACT_SILU):
+    """float32 x [M, K] times w [N, K]^T on FMA units (csrc/gemm_f32.cu): up to 8 rows by the kernel that streams w
+    once, more by tiles."""
+    M, K = x.shape
+    fn = core().tq_gemv_f32 if M <= F32_ROW_KERNEL_MAX_ROWS else core().tq_gemm_f32
+    check(fn(ptr(x), ptr(w), ptr(bias), ptr(out), M, out.shape[1], K, x.stride(0), w.stride(0), out.stride(0),
+             int(accumulate), _gate(swiglu, activation), stream()), "gemm_f32")
+    return out
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = None,
            out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
            accumulate: bool = False, swiglu: bool = False, activation: int = elementwise.ACT_SILU) -> torch.Tensor:
@@ -267,6 +289,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = N
         return decode_gemm_tc(x, w, out, bias, accumulate, swiglu, activation)
     if _skinny_ok(x, w):
         return skinny_gemm(x, w, out, bias, accumulate, swiglu, activation)
+    if _f32_ok(x, w, out):
+        return gemm_f32(x, w, out, bias, accumulate, swiglu, activation)
     if M <= ROW_KERNEL_MAX_ROWS:
         return gemv_rows(x, w, out, bias, accumulate, swiglu, activation)
 
