@@ -75,6 +75,14 @@ __device__ __forceinline__ float fd_tanh_cap(float x, float cap, float two_log2e
 // VT: 1 if the values have a tile of their own beside the keys' in every stage; 0 for a cache whose values are its
 // keys (one row per token, given as both arrays): the row is fetched once and read as both operands, and the
 // shared memory that saves goes into longer chunks.
+//
+// Rows of more than 128 entries (VT = 0 only: latents with their rotated part) would hold q's fragments and the sums of
+// all dims in 200 registers: q then lies in shared memory and is read by ldmatrix for every chunk.  These rows ran on
+// the general kernel before, which keeps the weights of the softmax in float32; they stay exact here as three bfloat16
+// parts whose products with the values are summed in float32 (p = p1 + p2 + p3 holds all 24 bits).  Bound by latency at
+// few tokens, by the tensor pipe (8 instructions a key, 6 of them for the values) at many.  Measured, rows of 256, 16
+// heads, launched from Python with the merge, general kernel -> this one: 1 token at 3,000 keys 102 -> 30 us, 64 tokens
+// at 2,000 keys 516 -> 48, 64 sequences continued by 77 tokens at 100 keys 2,220 -> 340.
 template <int HD, int FD_CHUNK, int WEIGHTS = FD_SOFTMAX, int VT = 1>
 __global__ void __launch_bounds__(FD_WARPS * 32)
 flash_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages, const bf16* __restrict__ v_pages,
@@ -90,6 +98,8 @@ flash_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages
     constexpr int TILE = FD_CHUNK * ROW;                   // one K or V chunk
     constexpr int TPS = VT ? 2 : 1;                        // tiles per stage
     constexpr int WARP_BYTES = FD_STAGES * TPS * TILE;
+    constexpr bool WIDE = HD > 128;                        // q in shared memory, weights in three parts
+    static_assert(!WIDE || (VT == 0 && WEIGHTS != FD_SIGMOID), "wide rows: a cache whose values are its keys");
     constexpr int KS = HD / 16;                            // k-steps of Q·K^T
     constexpr int NT = HD / 8;                             // n-tiles of P·V
     extern __shared__ __align__(16) unsigned char smem[];
@@ -170,9 +180,17 @@ flash_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages
     }
 
     // Q fragments: rows = q heads of this group (rows >= n_rep are zero)
-    uint32_t qf[KS][4];
-    {
-        const bf16* q0 = q + ((size_t)t * nh + (size_t)g * n_rep) * HD;
+    uint32_t qf[WIDE ? 1 : KS][4];
+    const bf16* q0 = q + ((size_t)t * nh + (size_t)g * n_rep) * HD;
+    unsigned char* q_sh = smem + FD_WARPS * WARP_BYTES;
+    if constexpr (WIDE) {
+        for (int p = threadIdx.x; p < 16 * PR; p += FD_WARPS * 32) {
+            const int r = p / PR, c = p - r * PR;
+            *reinterpret_cast<uint4*>(q_sh + r * ROW + c * 16) =
+                r < n_rep ? *reinterpret_cast<const uint4*>(q0 + (size_t)r * HD + c * 8) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        __syncthreads();
+    } else {
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
             const int d = ks * 16 + 2 * tid4;
@@ -198,13 +216,15 @@ flash_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages
         for (int n = 0; n < ST; ++n) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; }
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
+            uint32_t* qa = qf[WIDE ? 0 : ks];
+            if constexpr (WIDE) fd_ldmatrix_x4(qa, q_sh + (lane & 15) * ROW + (2 * ks + (lane >> 4)) * 16);
 #pragma unroll
             for (int n = 0; n < ST; n += 2) {
                 uint32_t kb[4];
                 const int mat = lane >> 3, r = lane & 7;
                 fd_ldmatrix_x4(kb, ks_ + ((n + (mat >> 1)) * 8 + r) * ROW + (2 * ks + (mat & 1)) * 16);
-                fd_mma(s[n], qf[ks], kb[0], kb[1]);
-                fd_mma(s[n + 1], qf[ks], kb[2], kb[3]);
+                fd_mma(s[n], qa, kb[0], kb[1]);
+                fd_mma(s[n + 1], qa, kb[2], kb[3]);
             }
         }
         float corr[2] = {1.f, 1.f};
@@ -284,16 +304,28 @@ flash_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages
         }
 #pragma unroll
         for (int kk = 0; kk < FD_CHUNK / 16; ++kk) {
-            const uint32_t pf[4] = {fd_pack(s[2 * kk][0], s[2 * kk][1]), fd_pack(s[2 * kk][2], s[2 * kk][3]),
-                                    fd_pack(s[2 * kk + 1][0], s[2 * kk + 1][1]),
-                                    fd_pack(s[2 * kk + 1][2], s[2 * kk + 1][3])};
+            constexpr int PARTS = WIDE ? 3 : 1;
+            uint32_t pf[PARTS][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float a = s[2 * kk + (e >> 1)][2 * (e & 1)], b = s[2 * kk + (e >> 1)][2 * (e & 1) + 1];
+#pragma unroll
+                for (int part = 0; part < PARTS; ++part) {
+                    pf[part][e] = fd_pack(a, b);
+                    a -= __uint_as_float(pf[part][e] << 16);       // what the part leaves (exact)
+                    b -= __uint_as_float(pf[part][e] & 0xffff0000u);
+                }
+            }
 #pragma unroll
             for (int n = 0; n < NT; n += 2) {
                 uint32_t vb[4];
                 const int mat = lane >> 3, r = lane & 7;
                 fd_ldmatrix_x4_trans(vb, vs_ + (kk * 16 + (mat & 1) * 8 + r) * ROW + (n + (mat >> 1)) * 16);
-                fd_mma(o[n], pf, vb[0], vb[1]);
-                fd_mma(o[n + 1], pf, vb[2], vb[3]);
+#pragma unroll
+                for (int part = PARTS - 1; part >= 0; --part) {    // the smallest first
+                    fd_mma(o[n], pf[part], vb[0], vb[1]);
+                    fd_mma(o[n + 1], pf[part], vb[2], vb[3]);
+                }
             }
         }
         __syncwarp();                                      // the stage may be overwritten by the next issue
@@ -381,8 +413,8 @@ static int launch_flash_decode(const bf16* q, const bf16* kp, const bf16* vp, co
                                const float* gate = nullptr, int ldg = 0, int kv_div = 1,
                                FdOptions opt = FdOptions{0.f, 0.f, nullptr, 0, nullptr, 0}) {
     constexpr int ROW = HD * 2 + 16;
-    constexpr int FD_CHUNK = (HD <= 64 || !VT) ? 32 : 16;
-    constexpr size_t stage_bytes = (size_t)FD_WARPS * FD_STAGES * (VT ? 2 : 1) * FD_CHUNK * ROW;
+    constexpr int FD_CHUNK = (HD <= 64 || (!VT && HD <= 128)) ? 32 : 16;
+    constexpr size_t stage_bytes = (size_t)FD_WARPS * FD_STAGES * (VT ? 2 : 1) * FD_CHUNK * ROW + (HD > 128 ? 16 * ROW : 0);
     constexpr size_t merge_bytes = (size_t)FD_WARPS * 16 * (HD + 2) * sizeof(float);
     constexpr size_t smem = stage_bytes > merge_bytes ? stage_bytes : merge_bytes;
     static bool configured[64] = {false};         // per device: the attribute belongs to the device's copy of the kernel
@@ -402,7 +434,7 @@ static int launch_flash_decode(const bf16* q, const bf16* kp, const bf16* vp, co
 }
 
 // Returns cudaErrorNotSupported (801) for shapes outside this kernel's reach
-// (head_dim not in {32, 64, 96, 128}, q heads per key/value head that do not
+// (head_dim not in {32, 64, 96, 128}, or in {192, 256} with values that are the keys; q heads per key/value head that do not
 // cut into equal groups of at most 16, pages of another size); the caller then uses the general kernel.
 //
 // `early_start`: launch the kernel so that it may begin while its predecessor in the stream still runs
@@ -436,6 +468,8 @@ static int flash_decode_launch(const void* q, const void* k_pages, const void* v
         TQ_FD(64);
         TQ_FD(96);
         TQ_FD(128);
+        case 192: return same ? launch_flash_decode<192, FD_SOFTMAX, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
+        case 256: return same ? launch_flash_decode<256, FD_SOFTMAX, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
         default: return (int)cudaErrorNotSupported;
     }
 #undef TQ_FD_ARGS
@@ -511,6 +545,8 @@ TQ_API int tq_flash_decode_ext(const void* q, const void* k_pages, const void* v
         TQ_FD(64);
         TQ_FD(96);
         TQ_FD(128);
+        case 192: return same ? launch_flash_decode<192, FD_SOFTMAX_EXT, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
+        case 256: return same ? launch_flash_decode<256, FD_SOFTMAX_EXT, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
         default: return (int)cudaErrorNotSupported;
     }
 #undef TQ_FD_ARGS

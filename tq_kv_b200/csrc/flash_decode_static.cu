@@ -76,7 +76,9 @@ int tq_flash_decode_static(const void* q, const void* k_pages, const void* v_pag
     }
     // Without an early start: whatever the caller ran before in this stream (a kernel that writes the positions,
     // the table or many keys) has completed before the first block reads anything.
-    int st = flash_decode_launch(q, k_pages, v_pages, block_table, table_width, ring_pages, page_tokens, tok_pos,
+    int st = (int)cudaErrorNotSupported;
+    if (head_dim <= 128)                                     // (the wide rows of shared latents are the engine's own)
+        st = flash_decode_launch(q, k_pages, v_pages, block_table, table_width, ring_pages, page_tokens, tok_pos,
                                  tok_seq, window, scale, out, part_acc, part_ml, n_tokens, n_heads, n_kv_heads,
                                  head_dim, n_splits, 0, stream);
     if (st == (int)cudaErrorNotSupported) {
