@@ -1,0 +1,132 @@
+"""The matrix-state scans over steps of many tokens, on both sides of the line between the kernel that goes eight tokens at
+a time (csrc/block_scan.cu) and the one that goes token by token (csrc/linear_scan.cu), against float64.  Bound: the sums
+of a token are a few hundred float32 terms and the state fades or is overwritten, so errors stay a few 1e-7 of the largest
+value; 2e-6 allows for the growth of undamped states."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def i32(x):
+    return torch.tensor(x, dtype=torch.int32, device=DEV)
+
+
+def make(mode, lens, H, G, d, e, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    T = sum(lens)
+
+    def rnd(*s):
+        return torch.randn(*s, generator=g, device=DEV)
+
+    p = {"q": rnd(T, G * d), "k": rnd(T, G * d), "v": rnd(T, H * e), "state": rnd(len(lens) + 2, H * d * e) * 0.3}
+    if mode == "delta":
+        p["a"], p["w"] = rnd(T, H * d), rnd(T, H * d) * 2
+    elif mode == "decay":
+        p["c"] = torch.linspace(0.5, 1.0, H, device=DEV)
+    else:
+        p["k"] = torch.nn.functional.normalize(p["k"].reshape(T, G, d), dim=-1).reshape(T, -1)
+        p["s"] = torch.rand(T, H, 4, generator=g, device=DEV)
+        p["s"][..., 0] = p["s"][..., 0] ** 0.2
+        p["skip"] = rnd(H)
+    return p
+
+
+def exact(mode, p, lens, slots, H, G, d, e):
+    T = sum(lens)
+    q, k, v = (p[n].double() for n in "qkv")
+    if mode == "decay":
+        q, k, v = (torch.nn.functional.silu(x) for x in (q, k, v))
+    q, k = (x.reshape(T, G, d).repeat_interleave(H // G, 1) for x in (q, k))
+    v = v.reshape(T, H, e)
+    out, state, t = torch.empty(T, H, e, dtype=torch.float64, device=DEV), p["state"].double().clone(), 0
+    if mode == "delta":
+        w = torch.exp(-math.exp(-0.5) * torch.sigmoid(p["w"].double())).reshape(T, H, d, 1)
+        u = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+        na = -(torch.sigmoid(p["a"].double()).reshape(T, H, d) * u)
+    for n, slot in zip(lens, slots):
+        S = state[slot].reshape(H, d, e)
+        for _ in range(n):
+            if mode == "delta":
+                r = (u[t].unsqueeze(1) @ S)
+                S = w[t] * S + na[t].unsqueeze(-1) * r + k[t].unsqueeze(-1) * v[t].unsqueeze(1)
+            elif mode == "decay":
+                S = p["c"].double().reshape(H, 1, 1) * S + k[t].unsqueeze(-1) * v[t].unsqueeze(1)
+            else:
+                S = p["s"][t, :, 0].double().reshape(H, 1, 1) * S
+                x = v[t] - (k[t].unsqueeze(1) @ S).squeeze(1) if mode == "gated_delta" else v[t]
+                S = S + k[t].unsqueeze(-1) * (p["s"][t, :, 1].double().unsqueeze(-1) * x).unsqueeze(1)
+            out[t] = (q[t].unsqueeze(1) @ S).squeeze(1)
+            if mode == "gated":
+                out[t] += p["skip"].double().unsqueeze(-1) * v[t]
+            t += 1
+        state[slot] = S.reshape(-1)
+    return out.reshape(T, H * e), state
+
+
+def run(mode, p, lens, slots, H, G, d, e):
+    from tq_kv_b200 import kernels
+    T, cu = sum(lens), [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    out, state = torch.full((T, H * e), float("nan"), device=DEV), p["state"].clone()
+    if mode in ("delta", "decay"):
+        cols = [p["q"], p["k"], p["v"]] + ([p["a"]] if mode == "delta" else [])
+        kw = dict(decay_logit=p["w"].clone(), off_a=2 * H * d + H * e) if mode == "delta" else dict(head_decay=p["c"], silu=True)
+        kernels.linear_scan(torch.cat(cols, 1), state.reshape(-1, H, d, e), i32(cu), i32(slots), out, n_seqs=len(lens), heads=H,
+                            key_dim=d, value_dim=e, off_q=0, off_k=H * d, off_v=2 * H * d, **kw)
+    else:
+        buf = torch.cat([p["q"], p["k"], p["v"]], 1)
+        kernels.gated_scan(buf[:, :G * d], buf[:, G * d:2 * G * d], buf[:, 2 * G * d:], p["s"], state, i32(cu), i32(slots), out,
+                           n_seqs=len(lens), heads=H, qk_heads=G, key_dim=d, value_dim=e, delta=mode == "gated_delta",
+                           skip=p["skip"] if mode == "gated" else None)
+    return out, state
+
+
+MODES = ["delta", "decay", "gated", "gated_delta"]
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("lens,H,G,d,e", [
+    ([1, 7, 8, 9, 16, 17, 40], 2, 2, 32, 32), ([70], 4, 2, 128, 128), ([33, 2], 3, 1, 64, 40), ([20, 31], 2, 1, 100, 12),
+    ([5, 64], 1, 1, 256, 20), ([9], 2, 2, 6, 132), ([25, 3], 32, 16, 128, 64),      # eight at a time, both forms
+    ([9] * 20, 2, 1, 128, 128), ([3, 30] * 30, 4, 4, 40, 24)])                      # token by token
+def test_against_float64(mode, lens, H, G, d, e):
+    if mode == "delta":
+        e = d
+    if mode in ("delta", "decay"):
+        G = H
+    slots = list(range(len(lens) + 1, 1, -1))
+    p = make(mode, lens, H, G, d, e, seed=d + e)
+    out, state = run(mode, p, lens, slots, H, G, d, e)
+    want, want_state = exact(mode, p, lens, slots, H, G, d, e)
+    for got, ref in ((out, want), (state, want_state)):
+        assert float((got.double() - ref).abs().max()) <= 2e-6 * float(ref.abs().max())
+    assert torch.equal(state[0], p["state"][0]) and torch.equal(state[1], p["state"][1])      # slots of no sequence
+
+
+@pytest.mark.parametrize("mode", ["delta", "gated"])
+def test_a_step_cut_into_pieces(mode):
+    """More records than one piece takes: the state waits in its slot between the pieces."""
+    from tq_kv_b200 import kernels
+    H, d, lens = 16, 128, [2500, 700]
+    assert kernels._lib.core().tq_scan_floats(1 if mode == "delta" else 2, sum(lens), 2, H, d, d) * 4 <= 100 << 20
+    p = make(mode, lens, H, H, d, d, seed=3)
+    out, state = run(mode, p, lens, [1, 3], H, H, d, d)
+    want, want_state = exact(mode, p, lens, [1, 3], H, H, d, d)
+    for got, ref in ((out, want), (state, want_state)):
+        assert float((got.double() - ref).abs().max()) <= 4e-6 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_a_token_changes_nothing_before_it(mode):
+    """An infinite value in a later token of the same eight leaves the results before it as they are."""
+    lens, H, d = [13], 2, 64
+    p = make(mode, lens, H, H, d, d, seed=5)
+    out, _ = run(mode, p, lens, [0], H, H, d, d)
+    p["v"][5] = float("inf")
+    spoiled, _ = run(mode, p, lens, [0], H, H, d, d)
+    assert torch.equal(out[:5], spoiled[:5]) and not torch.isfinite(spoiled[5]).any()

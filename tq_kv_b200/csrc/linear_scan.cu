@@ -18,7 +18,9 @@
 //   dt or beta; SCAN_CHANNEL_DELTA reads beta only), the value columns may be narrower or wider than the keys, and head h reads the q/k vectors of
 //   head h / qk_div.
 //
-// Everything here is float32: the state, and all that enters the recurrence.  Three kernels:
+// Everything here is float32: the state, and all that enters the recurrence.  Steps of many tokens of few sequences, which
+// the chain of tokens bounds, run eight tokens at a time (block_scan.cu, which also says where the line lies).  Three
+// kernels here:
 //
 // scan_prepare   once per (token, head), from the float32 results of the projections, in place:
 //                  SCAN_DELTA  decay logit -> w = exp(-exp(-1/2) * sigmoid(logit)); removal logit -> -(a * u)
@@ -38,40 +40,9 @@
 //                scan_prepare does for the scan), so a decode step is one launch.
 //                grid (sequence, head, column tile of 32).
 #include "common.cuh"
+#include "scan_modes.cuh"
 
-#define SCAN_DECAY 0
-#define SCAN_DELTA 1
-#define SCAN_GATED 2
-#define SCAN_GATED_DELTA 3
-#define SCAN_CHANNEL_DELTA 4
 #define SCAN_THREADS 128      // of the one-token kernel
-
-struct ScanArgs {
-    const float* q;           // [T, ldp] query vectors, head h at columns h*d (the pointers are already offset)
-    const float* k;           // keys, same layout
-    const float* v;           // values, head h at columns h*e
-    const float* au;          // SCAN_DELTA: minus removal rate times unit key (after scan_prepare)
-    int ldp;                  // row stride of q, k, v, au (one projection buffer)
-    const float* u;           // SCAN_DELTA: unit keys [T, ldu]
-    int ldu;
-    const float* w;           // SCAN_DELTA (after scan_prepare), SCAN_CHANNEL_DELTA: decay per key channel [T, ldw]
-    int ldw;
-    const float* head_decay;  // SCAN_DECAY: [H]
-    float* state;             // [slots, H, d, e]
-    const int* cu_seqlens;    // [B + 1] first token of each sequence in this step
-    const int* slots;         // [B]
-    float* out;               // [T, ldo], head h at columns h*e
-    int ldo;
-    int H, d, e;
-    int chunk;                // tokens staged at a time
-    int vec;                  // every vector starts on a 16-byte boundary and d, e are multiples of four
-    int silu;                 // linear_step, SCAN_DECAY: q, k, v pass through silu (nothing was prepared)
-    float unit_eps;           // linear_step, SCAN_DELTA: au and w hold the logits still (nothing was prepared)
-    const float* scal;        // SCAN_GATED*: [T, H, 4] per token and head: decay, then step size or write strength
-    const float* skip;        // SCAN_GATED: [H] or null, o += skip_head * v
-    int qk_div;               // head h reads the q/k vectors of head h / qk_div
-    size_t state_stride;      // floats from one slot's states to the next
-};
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float siluf_(float z) { return z / (1.f + expf(-z)); }
@@ -561,7 +532,7 @@ static int dispatch_step(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
 // every sequence brings exactly one token: one kernel then does everything and the buffers are left as they were.
 // Key widths up to 256.
 TQ_API int tq_linear_scan(int mode, float* q, float* k, float* v, float* a_logit, int ldp, float* w_logit, int ldw,
-                          float* u, int ldu, const float* head_decay, int silu, float unit_eps, float* state,
+                          float* u, int ldu, float* rec, const float* head_decay, int silu, float unit_eps, float* state,
                           const int* cu_seqlens, const int* slots, int n_seqs, int n_tokens, int single, float* out,
                           int ldo, int H, int d, int e, cudaStream_t stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
@@ -571,9 +542,11 @@ TQ_API int tq_linear_scan(int mode, float* q, float* k, float* v, float* a_logit
                silu, unit_eps, nullptr, nullptr, 1, (size_t)H * d * e};
     auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     a.vec = (d % 4 == 0 && e % 4 == 0 && ldp % 4 == 0 && al(q) && al(k) && al(v)) ? 1 : 0;
+    if (rec && !al(rec)) return (int)cudaErrorInvalidValue;
     if (mode == SCAN_DECAY) {
         if (!head_decay) return (int)cudaErrorInvalidValue;
         if (single) return dispatch_step<SCAN_DECAY>(a, n_seqs, stream);
+        if (rec) return block_scan(mode, a, n_seqs, n_tokens, rec, stream);
         if (silu) {
             const int threads = 256;
             for (int part = 0; part < 3; ++part) {
@@ -592,6 +565,7 @@ TQ_API int tq_linear_scan(int mode, float* q, float* k, float* v, float* a_logit
     if (mode == SCAN_DELTA) {
         if (!w_logit || !a_logit || e != d) return (int)cudaErrorInvalidValue;
         if (single) return dispatch_step<SCAN_DELTA>(a, n_seqs, stream);
+        if (rec) return block_scan(mode, a, n_seqs, n_tokens, rec, stream);
         if (!u) return (int)cudaErrorInvalidValue;
         a.vec = a.vec && ldu % 4 == 0 && ldw % 4 == 0 && al(u) && al(w_logit) && al(a_logit);
         const int rows = n_tokens * H;
@@ -603,14 +577,22 @@ TQ_API int tq_linear_scan(int mode, float* q, float* k, float* v, float* a_logit
     return (int)cudaErrorInvalidValue;
 }
 
+// Scratch of a step of many tokens, in floats: 0 if the token-by-token kernel takes it.  mode: 0, 1 as tq_linear_scan's;
+// 2, 3 tq_gated_scan without and with `delta`.
+TQ_API long long tq_scan_floats(int mode, int n_tokens, int n_seqs, int H, int d, int e) {
+    if (mode < 0 || mode > 3 || n_tokens <= 0 || n_seqs <= 0 || H <= 0 || d <= 0 || d > 256 || e <= 0) return 0;
+    return block_scan_floats(mode, n_tokens, n_seqs, H, d, e);
+}
+
 // The rules with one decay per head and token.  q, k [T, ldp] with H / qk_div heads of d, v [T, ldp] with H heads of
 // e, all in one float32 buffer and ready (activations, unit lengths and scales applied); scal [T, H, 4] holds each
 // token's decay and, with `delta`, its write strength beta (S' = g S; S = S' + k (beta (v - S'^T k))^T), else its
 // step size dt (S = g S + k (dt v)^T, o += skip_head * v if skip is given).  state points at the first slot's
-// [H, d, e] block; state_stride floats lie between slots.  `single`: one token per sequence.
+// [H, d, e] block; state_stride floats lie between slots.  `single`: one token per sequence.  rec: scratch of
+// tq_scan_floats(2 + delta, ...) floats where that is not 0.
 TQ_API int tq_gated_scan(int delta, const float* q, const float* k, const float* v, int ldp, const float* scal,
-                         const float* skip, int qk_div, float* state, long long state_stride, const int* cu_seqlens,
-                         const int* slots, int n_seqs, int n_tokens, int single, float* out, int ldo, int H, int d,
+                         const float* skip, int qk_div, float* rec, float* state, long long state_stride,
+                         const int* cu_seqlens, const int* slots, int n_seqs, int n_tokens, int single, float* out, int ldo, int H, int d,
                          int e, cudaStream_t stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
     if (!q || !k || !v || !scal || !state || !cu_seqlens || !slots || !out || H <= 0 || H > 65535 || d <= 0 || d > 256 ||
@@ -620,6 +602,8 @@ TQ_API int tq_gated_scan(int delta, const float* q, const float* k, const float*
                0, 0.f, scal, skip, qk_div, (size_t)state_stride};
     auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     a.vec = (d % 4 == 0 && e % 4 == 0 && ldp % 4 == 0 && al(q) && al(k) && al(v) && al(scal)) ? 1 : 0;
+    if (rec && !al(rec)) return (int)cudaErrorInvalidValue;
+    if (rec && !single) return block_scan(delta ? SCAN_GATED_DELTA : SCAN_GATED, a, n_seqs, n_tokens, rec, stream);
     if (delta) {
         if (single) return dispatch_step<SCAN_GATED_DELTA>(a, n_seqs, stream);
         return dispatch_scan<SCAN_GATED_DELTA>(a, n_seqs, stream);

@@ -184,7 +184,7 @@ _SIGNATURES = {
     "tq_embed_scaled": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_void_p],
     "tq_square_relu": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p],
     "tq_add_scaled": [c_void_p, c_void_p, c_size_t, c_float, c_void_p],
-    "tq_gated_scan": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, ctypes.c_longlong,
+    "tq_gated_scan": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, ctypes.c_longlong,
                       c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "tq_channel_delta_step": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
                               ctypes.c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
@@ -208,8 +208,8 @@ _SIGNATURES = {
     "tq_scale_inplace": [c_void_p, c_size_t, c_float, c_void_p],
     "tq_tanh_rows": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "tq_linear_scan": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
-                       c_int, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int,
-                       c_int, c_void_p],
+                       c_void_p, c_int, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int,
+                       c_int, c_int, c_void_p],
     "tq_rownorm_qkv_store": [c_void_p, c_int, c_void_p, c_void_p, c_float, c_float, c_int, c_void_p, c_void_p, c_void_p,
                              c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                              c_int, c_int, c_int, c_int, c_void_p],
@@ -288,6 +288,8 @@ def core() -> ctypes.CDLL:
             fn = getattr(lib, name)
             fn.argtypes = argtypes
             fn.restype = c_int
+        lib.tq_scan_floats.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int]
+        lib.tq_scan_floats.restype = ctypes.c_longlong
         lib.tq_channel_scan_floats.argtypes = [c_int, c_int, c_int, c_int]
         lib.tq_channel_scan_floats.restype = ctypes.c_longlong
         _core = lib

@@ -1,4 +1,4 @@
-"""Python entry point of the matrix-state recurrences (csrc/linear_scan.cu)."""
+"""Python entry point of the matrix-state recurrences (csrc/linear_scan.cu, csrc/block_scan.cu)."""
 from __future__ import annotations
 
 import ctypes
@@ -8,8 +8,14 @@ import torch
 
 from ._lib import KernelError, check, core, need_contiguous, ptr, stream
 
-SCAN_DECAY, SCAN_DELTA = 0, 1
+SCAN_DECAY, SCAN_DELTA, SCAN_GATED, SCAN_GATED_DELTA = 0, 1, 2, 3
 MAX_KEY_WIDTH = 256
+
+
+def _records(mode: int, n_tokens: int, n_seqs: int, heads: int, key_dim: int, value_dim: int, device) -> Optional[torch.Tensor]:
+    """Scratch of the scan that goes eight tokens at a time (csrc/block_scan.cu), None where the other kernel runs."""
+    n = core().tq_scan_floats(mode, n_tokens, int(n_seqs), heads, key_dim, value_dim)
+    return torch.empty(n, dtype=torch.float32, device=device) if n else None
 
 
 def linear_scan(proj: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor,
@@ -26,8 +32,8 @@ def linear_scan(proj: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tenso
     off_a of proj, the generalised delta rule:
         S_t = diag(w_t) S_{t-1} - (a_t * u_t)(u_t^T S_{t-1}) + k_t v_t^T,
         w = exp(-exp(-1/2) sigmoid(decay_logit)), a = sigmoid(removal logit), u = k / sqrt(|k|^2 + unit_eps).
-    Unless `single_tokens`, the kernels work in place: afterwards proj holds silu(q | k | v) (first rule, with `silu`) or -(a * u) in
-    place of the removal logits, and decay_logit holds w.  state float32 [slots, heads, d, e] is read at
+    Unless `single_tokens`, the kernels may work in place: afterwards proj may hold silu(q | k | v) (first rule, with `silu`) or -(a * u) in
+    place of the removal logits, and decay_logit w.  state float32 [slots, heads, d, e] is read at
     slots[b] before the first token and written after the last.  `single_tokens`: every sequence brings
     exactly one token (the kernel built for decoding runs)."""
     T, ld = proj.shape
@@ -47,15 +53,17 @@ def linear_scan(proj: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tenso
     if single_tokens and T != n_seqs:
         raise KernelError("linear_scan: single_tokens needs one token per sequence")
     need_contiguous(state=state, cu_seqlens=cu_seqlens, slots=slots, head_decay=head_decay)
-    u = a = None
+    u = a = rec = None
     ld_w = ld_u = 0
+    if not single_tokens:
+        rec = _records(SCAN_DECAY if decay_logit is None else SCAN_DELTA, T, n_seqs, heads, d, e, proj.device)
     if decay_logit is not None:
         if decay_logit.dtype != torch.float32 or tuple(decay_logit.shape) != (T, heads * d) or decay_logit.stride(1) != 1:
             raise KernelError("linear_scan: decay_logit must be float32 [T, heads * d]")
         if e != d or off_a + heads * d > ld:
             raise KernelError("linear_scan: the delta rule has square states; removal logits must fit the rows")
         mode, ld_w = SCAN_DELTA, decay_logit.stride(0)
-        if not single_tokens:
+        if not single_tokens and rec is None:
             u = torch.empty((T, heads * d), dtype=torch.float32, device=proj.device)
             ld_u = u.stride(0)
         a = proj[:, off_a:]
@@ -63,9 +71,9 @@ def linear_scan(proj: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tenso
         if head_decay.dtype != torch.float32 or head_decay.shape[0] != heads:
             raise KernelError("linear_scan: head_decay must be float32 [heads]")
         mode = SCAN_DECAY
-    n_kernels = 1 if single_tokens else (2 if mode == SCAN_DELTA else (4 if silu else 1))
+    n_kernels = 1 if single_tokens else (2 if rec is not None or mode == SCAN_DELTA else (4 if silu else 1))
     check(core().tq_linear_scan(mode, ptr(proj[:, off_q:]), ptr(proj[:, off_k:]), ptr(proj[:, off_v:]), ptr(a),
-                                proj.stride(0), ptr(decay_logit), ld_w, ptr(u), ld_u, ptr(head_decay), int(silu),
+                                proj.stride(0), ptr(decay_logit), ld_w, ptr(u), ld_u, ptr(rec), ptr(head_decay), int(silu),
                                 float(unit_eps), ptr(state), ptr(cu_seqlens), ptr(slots), int(n_seqs), T,
                                 int(single_tokens), ptr(out), out.stride(0), heads, d, e, stream()),
           "linear_scan", n_kernels)
@@ -151,7 +159,7 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scalars: torch
                cu_seqlens: torch.Tensor, slots: torch.Tensor, out: torch.Tensor, *, n_seqs: int, heads: int,
                qk_heads: int, key_dim: int, value_dim: int, delta: bool, skip: Optional[torch.Tensor] = None,
                single_tokens: bool = False):
-    """The matrix-state recurrences with one decay per head and token (csrc/linear_scan.cu).  q, k [T, qk_heads *
+    """The matrix-state recurrences with one decay per head and token (csrc/linear_scan.cu, csrc/block_scan.cu).  q, k [T, qk_heads *
     d] and v [T, heads * e] are column slices of ONE float32 buffer (one row stride), ready for the recurrence;
     head h reads the q/k vectors of head h // (heads // qk_heads).  scalars float32 [T, heads, 4] holds g and a
     second number per token and head.  With `delta`:  S' = g S;  S = S' + k (beta (v - S'^T k))^T  (second = beta);
@@ -176,9 +184,13 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scalars: torch
     if single_tokens and T != n_seqs:
         raise KernelError("gated_scan: single_tokens needs one token per sequence")
     need_contiguous(cu_seqlens=cu_seqlens, slots=slots, skip=skip)
+    rec = None
+    if not single_tokens:
+        rec = _records(SCAN_GATED_DELTA if delta else SCAN_GATED, T, n_seqs, heads, d, e, q.device)
     check(core().tq_gated_scan(int(bool(delta)), ptr(q), ptr(k), ptr(v), q.stride(0), ptr(scalars), ptr(skip),
-                               heads // qk_heads, ptr(state), state.stride(0), ptr(cu_seqlens), ptr(slots), int(n_seqs),
-                               T, int(single_tokens), ptr(out), out.stride(0), heads, d, e, stream()), "gated_scan")
+                               heads // qk_heads, ptr(rec), ptr(state), state.stride(0), ptr(cu_seqlens), ptr(slots),
+                               int(n_seqs), T, int(single_tokens), ptr(out), out.stride(0), heads, d, e, stream()),
+          "gated_scan", 1 if rec is None else 2)
     return out
 
 
