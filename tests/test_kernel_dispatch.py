@@ -32,3 +32,12 @@ def _w(n, k):
 ])
 def test_which_decode_kernel_takes_a_product(rows, n, k, swiglu, after_norm, f32, want):
     assert gemm._tc_takes(rows, _w(n, k), swiglu, after_norm, f32) is want
+
+
+@pytest.mark.parametrize("rows, n, k, swiglu, want", [
+    (1, 1152, 896, False, False), (1, 10304, 2048, False, True), (2, 10304, 2048, False, False),
+    (1, 2 * 5632, 2048, True, True), (1, 2 * 4864, 896, True, False), (1, 2 * 18944, 3584, True, False),
+    (1, 896, 4864, False, False), (1, 2048, 5632, False, True), (1, 3584, 18944, False, False),
+    (1, 151936, 896, False, True), (1, 152064, 3584, False, True), (2, 151936, 896, False, False)])
+def test_which_products_of_one_row_run_on_the_row_kernel(rows, n, k, swiglu, want):
+    assert gemm._row_takes(rows, _w(n, k), swiglu) is want

@@ -1,6 +1,8 @@
 """Matrix products: y = x · W^T with W stored [out, in].
 
 `linear()` picks the kernel from the operands:
+  * one row of bfloat16 and weights of middling size, or a head (`_row_takes`): the FMA
+    row kernel of csrc/row_gemm.cu;
   * up to 16 rows of bfloat16 and small weights (decoding a small model; the
     limits are in `_tc_takes`): the weight-streaming mma.sync kernel of
     csrc/skinny_gemm.cu, which reads the weight once and fuses bias, SwiGLU
@@ -98,6 +100,29 @@ def _tc_takes(rows: int, w: torch.Tensor, swiglu: bool, after_norm: bool, float3
     return size >= TC_DECODE_MIN_ADDED_BYTES or rows > TC_DECODE_ADDED_ROWS
 
 
+ROW_GEMM_MIN_BYTES = 16 << 20              # one row: products from this size
+ROW_GEMM_MIN_GATED_BYTES = 24 << 20        # (gated products from this one)
+ROW_GEMM_MAX_BYTES = 64 << 20              # up to this, beyond it only ...
+ROW_GEMM_HEAD_COLUMNS = 16384              # ... with so many columns
+
+
+def _row_takes(rows: int, w: torch.Tensor, swiglu: bool) -> bool:
+    """Which bfloat16 products of one row run on the FMA row kernel (csrc/row_gemm.cu), by the weight's size.  Measured in
+    whole passes of prompts and 24 decoded tokens, in ms, none / these / these without gated ones / without heads: 7B 72.4
+    / 71.0 / 70.7 / 71.6, zodosun-2k 20.2 / 18.7 / 19.4 / 18.9, rirudra-2k 9.73 / 8.72 / 9.00 / 9.05 (weights of 17 to
+    46 MB a product there, 26 and 33 MB in the 7B shape); given up to 24 MB only: 72.1 / 20.1 / 9.70.  Alone in replayed
+    graphs, in us: 9 MB 4.2 on the other kernel / 4.4 here, 23 MB 7.1 / 6.5, 26 MB 7.1 / 6.4, gated 17 MB 5.0 / 5.4,
+    gated 46 MB 11.7 / 10.3, 136 MB 23.9 / 23.6 (and in the 7B shape's step slower: its 3,584 long columns), a head of
+    272 MB 48.8 / 41.5.  With the norm made by the row kernel itself passes were slower (0.5B 15.9 -> 16.8 ms), two rows
+    gain little (a head 49.1 / 46.5) or lose (26 MB 7.0 / 8.7)."""
+    if rows != 1:
+        return False
+    size = w.numel() * 2
+    if not swiglu and w.shape[0] >= ROW_GEMM_HEAD_COLUMNS:
+        return size >= ROW_GEMM_MIN_BYTES
+    return (ROW_GEMM_MIN_GATED_BYTES if swiglu else ROW_GEMM_MIN_BYTES) <= size <= ROW_GEMM_MAX_BYTES
+
+
 def _gate(swiglu, activation) -> int:
     """The `swiglu` argument of the C functions: 0 for a plain product, ACT_SQUARE_RELU for a plain one with that
     activation on its result, else the gate's activation code."""
@@ -112,6 +137,13 @@ def skinny_gemm(x, w, out, bias=None, accumulate=False, swiglu=False, activation
     check(core().tq_skinny_gemm(ptr(x), ptr(w), ptr(bias), ptr(out), dtype_code(out), M, N, K, x.stride(0),
                                 w.stride(0), out.stride(0), int(accumulate), _gate(swiglu, activation), stream()),
           "skinny_gemm")
+    return out
+
+
+def row_gemm(x, w, out, bias=None, accumulate=False, swiglu=False, activation=elementwise.ACT_SILU):
+    """bfloat16 x [1, K] times bfloat16 w [N, K]^T on FMA units, streaming w once (csrc/row_gemm.cu); K a multiple of 8."""
+    check(core().tq_row_gemm(ptr(x), ptr(w), ptr(bias), ptr(out), dtype_code(out), out.shape[1], x.shape[1], w.stride(0),
+                             int(accumulate), _gate(swiglu, activation), stream()), "row_gemm")
     return out
 
 
@@ -155,6 +187,8 @@ def _fused_norm(x: "PendingNorm", w, out, bias, accumulate, swiglu, activation=e
     """Runs out (=, +=) norm(h) . w^T with the norm folded into a decode product; False if none takes it."""
     h, g = x.h, x.weight
     M, K = h.shape
+    if FUSE_NORM == "auto" and _row_takes(M, w, bool(swiglu)):
+        return False                                                          # the FMA row kernel's case
     big = _tc_takes(M, w, bool(swiglu), True, out.dtype == torch.float32)     # the tcgen05 kernel's case
     # Measured inside whole decode steps: the tcgen05 kernel gains from the folded norm where it runs in its
     # cluster form anyway (gated products: 7B shape -0.8 % of a step) and loses where the norm costs it the
@@ -188,6 +222,8 @@ def product_adds_shares(rows: int, w: torch.Tensor, after_norm: bool = True) -> 
     if not (USE_TCGEN05 and w.dtype == torch.bfloat16 and 0 < rows <= SKINNY_MAX_ROWS and K % 8 == 0
             and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0):
         return False
+    if _row_takes(rows, w, False):
+        return False                                   # the FMA row kernel takes it
     if not _tc_takes(rows, w, False, after_norm, True):
         return False                                   # the mma.sync kernel takes it
     return bool(core().tq_decode_gemm_tc_adds_shares(N, K))
@@ -281,6 +317,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = N
             return out
         x = pending.materialize()
 
+    if (_row_takes(M, w, bool(swiglu)) and USE_TCGEN05 and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K % 8 == 0
+            and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+            and out.dtype in (torch.float32, torch.bfloat16) and (not accumulate or out.dtype == torch.float32)):
+        return row_gemm(x, w, out, bias, accumulate, swiglu, activation)
     # decoding: the TMA-fed tcgen05 kernel or the mma.sync kernel (_tc_takes says which, where both can)
     if (USE_TCGEN05 and M <= SKINNY_MAX_ROWS and _tc_ok(x, w, out, swiglu)
             and (not accumulate or out.dtype == torch.float32) and not (relu2 and out.dtype != torch.bfloat16)
