@@ -19,7 +19,7 @@
 // the softmax's denominator (in the merge step where the keys are split).
 #include "common.cuh"
 
-#define ATT_MAX_PAIRS 8   // head_dim <= 512: each lane owns up to 8 pairs of dims
+#define ATT_MAX_PAIRS 8   // head_dim <= 512: each lane owns up to 8 pairs of dims (1, 2, 4 or 8: PAIRS below)
 
 struct KVSource {
     // packed: rows of this step, [T, nkv, hd]; key at position j of row b is token cu[b] + j - start[b]
@@ -61,8 +61,10 @@ __device__ __forceinline__ void kv_rows(const KVSource& src, int b, int j, int g
 }
 
 // grid (token, kv head, split); block = n_warps warps, warp w serves q heads
-// g*n_rep + w, + n_warps, ...
-template <typename TC>
+// g*n_rep + w, + n_warps, ...  Bound by the latency of its loads: a chunk's 32 keys are one dot product a lane, and the
+// value rows are asked for AHEAD at a time before the first is needed (they were waited for one by one).  Measured in
+// whole passes: 0.5B float32, two prompts of 150, 15 decoded tokens and their scoring 43.5 -> 39.5 ms.
+template <typename TC, int PAIRS>
 __global__ void attention_kernel(const TC* __restrict__ q, KVSource src, const int* __restrict__ tok_pos,
                                  const int* __restrict__ tok_seq, const int* __restrict__ cu_seqlens,
                                  const int* __restrict__ start_pos, int window, float scale, TC* __restrict__ out,
@@ -91,6 +93,7 @@ __global__ void attention_kernel(const TC* __restrict__ q, KVSource src, const i
     }
     float* qs = q_sh + warp * hd;
     constexpr int VEC = Vec16<TC>::N;
+    constexpr int AHEAD = PAIRS == 1 ? 16 : 16 / PAIRS;
 
     for (int hr = warp; hr < n_rep; hr += n_warps) {
         const int h = g * n_rep + hr;
@@ -100,9 +103,9 @@ __global__ void attention_kernel(const TC* __restrict__ q, KVSource src, const i
         __syncwarp();
 
         float m = -INFINITY, l = 0.f;
-        float acc[2 * ATT_MAX_PAIRS];
+        float acc[2 * PAIRS];
 #pragma unroll
-        for (int i = 0; i < 2 * ATT_MAX_PAIRS; ++i) acc[i] = 0.f;
+        for (int i = 0; i < 2 * PAIRS; ++i) acc[i] = 0.f;
 
         for (int base = lo; base < hi; base += 32) {
             const int c = base + lane;
@@ -113,6 +116,7 @@ __global__ void attention_kernel(const TC* __restrict__ q, KVSource src, const i
             if (valid) {
                 kv_rows<TC>(src, b, j, g, nkv, hd, vd, tok0, krow, vrow);
                 float dot = 0.f;
+#pragma unroll 8
                 for (int d = 0; d < hd; d += VEC) {
                     float kv[VEC];
                     load16_f32<TC>(krow + d, kv);
@@ -128,19 +132,30 @@ __global__ void attention_kernel(const TC* __restrict__ q, KVSource src, const i
             const float corr = expf(m - m_new);               // exp(-inf) = 0 on the first chunk
             l = l * corr + warp_sum(p);
 #pragma unroll
-            for (int i = 0; i < 2 * ATT_MAX_PAIRS; ++i) acc[i] *= corr;
+            for (int i = 0; i < 2 * PAIRS; ++i) acc[i] *= corr;
             m = m_new;
             const int n_here = min(32, hi - base);
-            for (int jj = 0; jj < n_here; ++jj) {
-                const float pj = __shfl_sync(0xffffffffu, p, jj);
-                const TC* vr = (const TC*)__shfl_sync(0xffffffffu, (unsigned long long)vrow, jj);
+            for (int j0 = 0; j0 < n_here; j0 += AHEAD) {
+                float2 vv[AHEAD][PAIRS];
 #pragma unroll
-                for (int i = 0; i < ATT_MAX_PAIRS; ++i) {
-                    const int d = 2 * lane + 64 * i;
-                    if (d < vd) {
-                        const float2 vv = load2_f32<TC>(vr + d);
-                        acc[2 * i] = fmaf(pj, vv.x, acc[2 * i]);
-                        acc[2 * i + 1] = fmaf(pj, vv.y, acc[2 * i + 1]);
+                for (int u = 0; u < AHEAD; ++u) {
+                    const TC* vr = (const TC*)__shfl_sync(0xffffffffu, (unsigned long long)vrow, j0 + u);
+#pragma unroll
+                    for (int i = 0; i < PAIRS; ++i) {
+                        const int d = 2 * lane + 64 * i;
+                        if (j0 + u < n_here && d < vd) vv[u][i] = load2_f32<TC>(vr + d);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) {
+                    const float pj = __shfl_sync(0xffffffffu, p, j0 + u);
+                    if (j0 + u >= n_here) continue;
+#pragma unroll
+                    for (int i = 0; i < PAIRS; ++i) {
+                        if (2 * lane + 64 * i < vd) {
+                            acc[2 * i] = fmaf(pj, vv[u][i].x, acc[2 * i]);
+                            acc[2 * i + 1] = fmaf(pj, vv[u][i].y, acc[2 * i + 1]);
+                        }
                     }
                 }
             }
@@ -153,12 +168,12 @@ __global__ void attention_kernel(const TC* __restrict__ q, KVSource src, const i
                 const float corr = expf(m - m_new);
                 l = l * corr + expf(sink - m_new);
 #pragma unroll
-                for (int i = 0; i < 2 * ATT_MAX_PAIRS; ++i) acc[i] *= corr;
+                for (int i = 0; i < 2 * PAIRS; ++i) acc[i] *= corr;
             }
             const float inv = 1.f / l;
             TC* o = out + ((size_t)t * nh + h) * vd;
 #pragma unroll
-            for (int i = 0; i < ATT_MAX_PAIRS; ++i) {
+            for (int i = 0; i < PAIRS; ++i) {
                 const int d = 2 * lane + 64 * i;
                 if (d < vd) store2_f32<TC>(o + d, acc[2 * i] * inv, acc[2 * i + 1] * inv);
             }
@@ -166,7 +181,7 @@ __global__ void attention_kernel(const TC* __restrict__ q, KVSource src, const i
             const size_t r = ((size_t)t * nh + h) * n_splits + split;
             float* pa = part_acc + r * vd;
 #pragma unroll
-            for (int i = 0; i < ATT_MAX_PAIRS; ++i) {
+            for (int i = 0; i < PAIRS; ++i) {
                 const int d = 2 * lane + 64 * i;
                 if (d < vd) store2_f32<float>(pa + d, acc[2 * i], acc[2 * i + 1]);
             }
@@ -175,42 +190,87 @@ __global__ void attention_kernel(const TC* __restrict__ q, KVSource src, const i
     }
 }
 
-// Merges the splits of one (token, head): grid (token, head), block 128.
-// Splits are combined in index order, so the result does not depend on
-// scheduling.  An empty split has m = -inf and l = 0 and contributes nothing.
+// Merges the splits of one (token, head): grid (token, head).  Bound by latency: a thread takes 16 bytes of the row and
+// every G-th split (G groups, about one for four splits), and asks for its first eight before it looks at the maxima, so
+// that up to 64 splits of a row of 128 arrive together (with the 128 threads of before, each walking all splits, 48 of them
+// took 10 us a layer; rirudra-2k, 24 tokens after a prompt of 3,000, 24 to 36 splits of 256: 8.70 -> 8.51 ms a pass); the groups meet in shared memory.  Splits are combined in a fixed order, so the
+// result does not depend on scheduling.  An empty split has m = -inf and l = 0 and contributes nothing.
+#define AM_THREADS 256
+#define AM_AHEAD 8
 template <typename TC>
-__global__ void attention_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
-                                       TC* __restrict__ out, int nh, int hd, int n_splits,
-                                       const float* __restrict__ sinks) {
+__global__ void __launch_bounds__(AM_THREADS)
+attention_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, TC* __restrict__ out, int nh,
+                       int hd, int n_splits, int piece_threads, const float* __restrict__ sinks) {
+    __shared__ float4 sums[AM_THREADS];
     const size_t r0 = ((size_t)blockIdx.x * nh + blockIdx.y) * n_splits;
     const int lane = threadIdx.x & 31;
+    const int piece = threadIdx.x % piece_threads, group = threadIdx.x / piece_threads, groups = blockDim.x / piece_threads;
+    const bool active = piece * 4 < hd;
+    const float* acc = part_acc + r0 * hd + piece * 4;
+    const float* ml = part_ml + 2 * r0;
+    const bool aligned = (reinterpret_cast<uintptr_t>(part_acc) & 15) == 0;      // (hd is a multiple of 8)
+    auto row = [&](int s) {
+        const float* x = acc + (size_t)s * hd;
+        return aligned ? *reinterpret_cast<const float4*>(x) : make_float4(x[0], x[1], x[2], x[3]);
+    };
     pdl_wait();
     pdl_launch();
+    float4 v[AM_AHEAD];
+    float ms[AM_AHEAD];
+#pragma unroll
+    for (int i = 0; i < AM_AHEAD; ++i) {
+        const int s = group + i * groups;
+        const bool on = active && s < n_splits;
+        v[i] = on ? row(s) : make_float4(0.f, 0.f, 0.f, 0.f);
+        ms[i] = on ? ml[2 * s] : -INFINITY;
+    }
     // every warp finds the maximum and the sum for itself, its lanes striding over the splits
     float m = -INFINITY;
-    for (int s = lane; s < n_splits; s += 32) m = fmaxf(m, part_ml[2 * (r0 + s)]);
+    for (int s = lane; s < n_splits; s += 32) m = fmaxf(m, ml[2 * s]);
     m = warp_max(m);
     const float sink = sinks ? sinks[blockIdx.y] : 0.f;
     if (sinks) m = fmaxf(m, sink);                  // the sink is one more split: maximum `sink`, sum 1, no values
     float l = 0.f;
     for (int s = lane; s < n_splits; s += 32) {
-        const float ms = part_ml[2 * (r0 + s)];
-        if (ms > -INFINITY) l += part_ml[2 * (r0 + s) + 1] * expf(ms - m);
+        const float mx = ml[2 * s];
+        if (mx > -INFINITY) l += ml[2 * s + 1] * expf(mx - m);
     }
     l = warp_sum(l);
     if (sinks) l += expf(sink - m);
-    TC* o = out + ((size_t)blockIdx.x * nh + blockIdx.y) * hd;
-    for (int d = threadIdx.x; d < hd; d += blockDim.x) {
-        float a = 0.f;
-        // the loads do not wait for one another: a split without keys is dropped after its load, not around it
-#pragma unroll 4
-        for (int s = 0; s < n_splits; ++s) {
-            const float ms = part_ml[2 * (r0 + s)];
-            const float v = part_acc[(r0 + s) * hd + d];
-            a += ms > -INFINITY ? v * expf(ms - m) : 0.f;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](const float4& x, float mx) {     // (a split without keys is dropped: whatever its row holds)
+        if (mx > -INFINITY) {
+            const float f = expf(mx - m);
+            a.x = fmaf(x.x, f, a.x); a.y = fmaf(x.y, f, a.y); a.z = fmaf(x.z, f, a.z); a.w = fmaf(x.w, f, a.w);
         }
-        o[d] = from_f32<TC>(a / l);
+    };
+#pragma unroll
+    for (int i = 0; i < AM_AHEAD; ++i) add(v[i], ms[i]);
+    for (int s = group + AM_AHEAD * groups; s < n_splits; s += groups)
+        if (active) add(row(s), ml[2 * s]);
+    sums[threadIdx.x] = a;
+    __syncthreads();
+    if (group == 0 && active) {
+        for (int g = 1; g < groups; ++g) {
+            const float4 x = sums[g * piece_threads + piece];
+            a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+        }
+        TC* o = out + ((size_t)blockIdx.x * nh + blockIdx.y) * hd + piece * 4;
+        store2_f32<TC>(o, a.x / l, a.y / l);
+        store2_f32<TC>(o + 2, a.z / l, a.w / l);
     }
+}
+
+// Threads a row of hd values takes, 16 bytes each (a power of two), and those of a block.
+static int merge_piece_threads(int hd) {
+    int n = 8;
+    while (n * 4 < hd) n *= 2;
+    return n;
+}
+static int merge_threads(int pt, int n_splits) {
+    int n = pt < 32 ? 32 : pt;
+    while (n * 2 <= AM_THREADS && n / pt * 4 < n_splits) n *= 2;
+    return n;
 }
 
 // Scratch needed for n_splits > 1: part_acc float[T*nh*n_splits*vd], part_ml float[T*nh*n_splits*2].  Without `out`
@@ -237,23 +297,30 @@ TQ_API int tq_attention_ext(const void* q, int dtype, const void* k_packed, cons
     const int n_warps = n_rep < 8 ? n_rep : 8;
     const dim3 grid(n_tokens, nkv, n_splits);
     const size_t smem = (size_t)n_warps * hd * sizeof(float);
-    if (dtype == TQ_F32)
-        attention_kernel<float><<<grid, n_warps * 32, smem, stream>>>(
-            (const float*)q, src, tok_pos, tok_seq, cu_seqlens, start_pos, window, scale, (float*)out, part_acc,
-            part_ml, nh, nkv, hd, n_splits, opt);
-    else if (dtype == TQ_BF16)
-        attention_kernel<bf16><<<grid, n_warps * 32, smem, stream>>>(
-            (const bf16*)q, src, tok_pos, tok_seq, cu_seqlens, start_pos, window, scale, (bf16*)out, part_acc,
-            part_ml, nh, nkv, hd, n_splits, opt);
-    else
-        return (int)cudaErrorInvalidValue;
+#define TQ_ATT(TC, P)                                                                                                      \
+    attention_kernel<TC, P><<<grid, n_warps * 32, smem, stream>>>((const TC*)q, src, tok_pos, tok_seq, cu_seqlens, start_pos, \
+                                                                  window, scale, (TC*)out, part_acc, part_ml, nh, nkv, hd,    \
+                                                                  n_splits, opt)
+#define TQ_ATT_PAIRS(TC)                    \
+    do {                                    \
+        if (vd <= 64) TQ_ATT(TC, 1);        \
+        else if (vd <= 128) TQ_ATT(TC, 2);  \
+        else if (vd <= 256) TQ_ATT(TC, 4);  \
+        else TQ_ATT(TC, 8);                 \
+    } while (0)
+    if (dtype == TQ_F32) TQ_ATT_PAIRS(float);
+    else if (dtype == TQ_BF16) TQ_ATT_PAIRS(bf16);
+    else return (int)cudaErrorInvalidValue;
+#undef TQ_ATT_PAIRS
+#undef TQ_ATT
     int st = tq_launch_status();
     if (st || !part_acc || !out) return st;
     const dim3 mgrid(n_tokens, nh);
+    const int pt = merge_piece_threads(vd), threads = merge_threads(pt, n_splits);
     if (dtype == TQ_F32)
-        attention_merge_kernel<float><<<mgrid, 128, 0, stream>>>(part_acc, part_ml, (float*)out, nh, vd, n_splits, sinks);
+        attention_merge_kernel<float><<<mgrid, threads, 0, stream>>>(part_acc, part_ml, (float*)out, nh, vd, n_splits, pt, sinks);
     else
-        attention_merge_kernel<bf16><<<mgrid, 128, 0, stream>>>(part_acc, part_ml, (bf16*)out, nh, vd, n_splits, sinks);
+        attention_merge_kernel<bf16><<<mgrid, threads, 0, stream>>>(part_acc, part_ml, (bf16*)out, nh, vd, n_splits, pt, sinks);
     return tq_launch_status();
 }
 
@@ -272,13 +339,14 @@ TQ_API int tq_attention(const void* q, int dtype, const void* k_packed, const vo
 TQ_API int tq_attention_merge(const float* part_acc, const float* part_ml, void* out, int dtype, int n_tokens, int nh,
                               int hd, int n_splits, const float* sinks, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
-    if (n_splits < 1 || !part_acc || !part_ml) return (int)cudaErrorInvalidValue;
+    if (n_splits < 1 || !part_acc || !part_ml || hd <= 0 || hd % 8 || hd > 64 * ATT_MAX_PAIRS) return (int)cudaErrorInvalidValue;
     const dim3 mgrid(n_tokens, nh);
+    const int pt = merge_piece_threads(hd), threads = merge_threads(pt, n_splits);
     if (dtype == TQ_F32)
-        return tq_launch_pdl(TQ_PDL_MERGE, attention_merge_kernel<float>, mgrid, dim3(128), 0, stream, part_acc, part_ml,
-                             (float*)out, nh, hd, n_splits, sinks);
+        return tq_launch_pdl(TQ_PDL_MERGE, attention_merge_kernel<float>, mgrid, dim3(threads), 0, stream, part_acc, part_ml,
+                             (float*)out, nh, hd, n_splits, pt, sinks);
     if (dtype == TQ_BF16)
-        return tq_launch_pdl(TQ_PDL_MERGE, attention_merge_kernel<bf16>, mgrid, dim3(128), 0, stream, part_acc, part_ml,
-                             (bf16*)out, nh, hd, n_splits, sinks);
+        return tq_launch_pdl(TQ_PDL_MERGE, attention_merge_kernel<bf16>, mgrid, dim3(threads), 0, stream, part_acc, part_ml,
+                             (bf16*)out, nh, hd, n_splits, pt, sinks);
     return (int)cudaErrorInvalidValue;
 }
