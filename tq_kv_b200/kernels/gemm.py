@@ -76,6 +76,7 @@ SKINNY_MAX_ROWS = 64
 # Weights from which a decode product of up to 16 rows runs on the tcgen05 kernel (see _tc_takes)
 TC_DECODE_MIN_WEIGHT_BYTES = 24 << 20      # the product after a pending norm
 TC_DECODE_MIN_GATED_BYTES = 64 << 20       # gated products
+TC_DECODE_GATED_ROWS = 8                   # ... and these from 9 rows on at any size
 TC_DECODE_MIN_ADDED_BYTES = 4 << 20        # float32 results of given rows, which leave as shares of K
 TC_DECODE_ADDED_ROWS = 8                   # ... and these from 9 rows on at any size
 
@@ -94,7 +95,7 @@ def _tc_takes(rows: int, w: torch.Tensor, swiglu: bool, after_norm: bool, float3
         return True
     size = w.numel() * 2
     if swiglu:
-        return size >= TC_DECODE_MIN_GATED_BYTES
+        return size >= TC_DECODE_MIN_GATED_BYTES or rows > TC_DECODE_GATED_ROWS
     if after_norm or not float32_out:
         return size >= TC_DECODE_MIN_WEIGHT_BYTES
     return size >= TC_DECODE_MIN_ADDED_BYTES or rows > TC_DECODE_ADDED_ROWS
@@ -194,7 +195,8 @@ def _fused_norm(x: "PendingNorm", w, out, bias, accumulate, swiglu, activation=e
     # cluster form anyway (gated products: 7B shape -0.8 % of a step) and loses where the norm costs it the
     # form with independent shares of K (float32 results: +8 %); the mma.sync kernel gains for plain products
     # (0.5B shape -1.5 %) and loses for gated ones, whose registers are scarce (+2 %).
-    if FUSE_NORM == "auto" and big != bool(swiglu):
+    # (Gated products below 64 MB of 9 to 16 rows: 46 MB 18.0 with the fold, 15.6 and a norm kernel of 2 without.)
+    if FUSE_NORM == "auto" and (big != bool(swiglu) or (swiglu and w.numel() * 2 < TC_DECODE_MIN_GATED_BYTES)):
         return False
     if not (FUSE_NORM and USE_TCGEN05 and x.out_dtype == torch.bfloat16 and w.dtype == torch.bfloat16
             and h.dtype == torch.float32 and g.dtype == torch.float32 and 0 < M <= FUSED_NORM_MAX_ROWS
