@@ -410,12 +410,17 @@ static int dispatch_scan(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
 }
 
 // ---------------------------------------------------------------------------
-// linear_step: one token per sequence.  Warp w of a block owns keys w, w + 4, ... and 32 columns; partial dot
-// products meet in shared memory.  The token's vectors are staged once per block.
+// linear_step: one token per sequence.  Warp w of a block owns a quarter of the keys and 32 columns; partial dot
+// products meet in shared memory.  The token's vectors are staged once per block and read four keys at a time.
 // ---------------------------------------------------------------------------
 #define SCAN_STEP_VECTORS(MODE) ((MODE) == SCAN_DELTA ? 5 : ((MODE) == SCAN_CHANNEL_DELTA ? 4 : 2))
+// Blocks an SM, by rule: as many as leave the state's registers unspilled.  Measured in replayed graphs, 64 sequences, 16
+// heads of 128 x 128 (134 MB read and written), in us, four blocks of 128 registers and one key a load before / now: delta
+// rule 39.6 / 35.7, constant decay 34.2 / 28.2, one decay with the delta rule 42.0 / 31.8 (floor 20.5).
+#define SCAN_STEP_BLOCKS(MODE) ((MODE) == SCAN_DECAY ? 8 : ((MODE) == SCAN_GATED_DELTA ? 6 : ((MODE) == SCAN_DELTA ? 5 : 4)))
 template <int MODE, int KPW>      // KPW: keys per warp (d <= 4 * KPW)
-__global__ void __launch_bounds__(SCAN_THREADS) linear_step_kernel(ScanArgs a) {
+__global__ void __launch_bounds__(SCAN_THREADS, KPW <= 32 ? SCAN_STEP_BLOCKS(MODE) : 1) linear_step_kernel(ScanArgs a) {
+    constexpr int DP = 4 * KPW;                               // the vectors' keys from d on are zeros
     extern __shared__ __align__(16) float sm[];
     const int b = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
@@ -423,11 +428,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) linear_step_kernel(ScanArgs a) {
     const int hq = head / a.qk_div;
     const bool col_ok = col < e;
     float* sq = sm;                 // [d] each: q k (u au w; or the products w k in u's place, then w)
-    float* sk = sq + d;
-    float* su = sk + d;
-    float* sau = su + d;
-    float* sw = MODE == SCAN_CHANNEL_DELTA ? sau : sau + d;
-    float* red = sm + SCAN_STEP_VECTORS(MODE) * d;            // [4] + pad, then [2][4][32]
+    float* sk = sq + DP;
+    float* su = sk + DP;
+    float* sau = su + DP;
+    float* sw = MODE == SCAN_CHANNEL_DELTA ? sau : sau + DP;
+    float* red = sm + SCAN_STEP_VECTORS(MODE) * DP;           // [4] + pad, then [2][4][32]
     pdl_wait();
     pdl_launch();
     const int t = a.cu_seqlens[b];
@@ -436,12 +441,18 @@ __global__ void __launch_bounds__(SCAN_THREADS) linear_step_kernel(ScanArgs a) {
     float S[KPW];
 #pragma unroll
     for (int i = 0; i < KPW; ++i) {
-        const int key = i * 4 + warp;
+        const int key = warp * KPW + i;
         S[i] = (col_ok && key < d) ? st[(size_t)key * e + col] : 0.f;
     }
     // the token's vectors, made here from the projections' results (one token: no prepare kernel runs before)
     float ss = 0.f;
-    for (int i = tid; i < d; i += SCAN_THREADS) {
+    for (int i = tid; i < DP; i += SCAN_THREADS) {
+        if (i >= d) {
+            sq[i] = sk[i] = 0.f;
+            if (MODE == SCAN_DELTA) su[i] = sau[i] = sw[i] = 0.f;
+            if (MODE == SCAN_CHANNEL_DELTA) su[i] = sw[i] = 0.f;
+            continue;
+        }
         float qv = a.q[(size_t)t * a.ldp + hq * d + i], kv = a.k[(size_t)t * a.ldp + hq * d + i];
         if (MODE == SCAN_DECAY && a.silu) { qv = siluf_(qv); kv = siluf_(kv); }
         sq[i] = qv;
@@ -478,11 +489,14 @@ __global__ void __launch_bounds__(SCAN_THREADS) linear_step_kernel(ScanArgs a) {
         s2 = a.scal[((size_t)t * a.H + head) * 4 + 1];
     }
     if (MODE == SCAN_DELTA || MODE == SCAN_GATED_DELTA || MODE == SCAN_CHANNEL_DELTA) {
-        const float* sd = MODE == SCAN_GATED_DELTA ? sk : su;
+        const float4* sd = reinterpret_cast<const float4*>((MODE == SCAN_GATED_DELTA ? sk : su) + warp * KPW);
 #pragma unroll
-        for (int i = 0; i < KPW; ++i) {
-            const int key = i * 4 + warp;
-            if (key < d) dot = fmaf(sd[key], S[i], dot);
+        for (int i = 0; i < KPW / 4; ++i) {
+            const float4 x = sd[i];
+            dot = fmaf(x.x, S[4 * i], dot);
+            dot = fmaf(x.y, S[4 * i + 1], dot);
+            dot = fmaf(x.z, S[4 * i + 2], dot);
+            dot = fmaf(x.w, S[4 * i + 3], dot);
         }
         red[128 + warp * 32 + lane] = dot;
         __syncthreads();
@@ -494,15 +508,23 @@ __global__ void __launch_bounds__(SCAN_THREADS) linear_step_kernel(ScanArgs a) {
     if (MODE == SCAN_GATED) vw = s2 * vj;
     if (MODE == SCAN_GATED_DELTA) vw = s2 * (vj - g * dot);
     if (MODE == SCAN_CHANNEL_DELTA) vw = s2 * (vj - dot);
+    float* row = st + (size_t)warp * KPW * e + col;
 #pragma unroll
-    for (int i = 0; i < KPW; ++i) {
-        const int key = i * 4 + warp;
-        if (key < d) {
-            if (MODE == SCAN_DELTA) S[i] = fmaf(sw[key], S[i], fmaf(sk[key], vj, sau[key] * dot));
-            else if (MODE == SCAN_CHANNEL_DELTA) S[i] = fmaf(sw[key], S[i], sk[key] * vw);
-            else S[i] = fmaf(c_head, S[i], sk[key] * vw);
-            o = fmaf(sq[key], S[i], o);
-            if (col_ok) st[(size_t)key * e + col] = S[i];
+    for (int i = 0; i < KPW / 4; ++i) {
+        const int key = warp * KPW + 4 * i;
+        const float4 k4 = *reinterpret_cast<const float4*>(sk + key), q4 = *reinterpret_cast<const float4*>(sq + key);
+        float4 w4 = make_float4(c_head, c_head, c_head, c_head), a4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (MODE == SCAN_DELTA || MODE == SCAN_CHANNEL_DELTA) w4 = *reinterpret_cast<const float4*>(sw + key);
+        if (MODE == SCAN_DELTA) a4 = *reinterpret_cast<const float4*>(sau + key);
+        const float kk[4] = {k4.x, k4.y, k4.z, k4.w}, qq[4] = {q4.x, q4.y, q4.z, q4.w}, ww[4] = {w4.x, w4.y, w4.z, w4.w},
+                    aa[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            float v = S[4 * i + x];
+            if (MODE == SCAN_DELTA) v = fmaf(ww[x], v, fmaf(kk[x], vj, aa[x] * dot));
+            else v = fmaf(ww[x], v, kk[x] * vw);
+            o = fmaf(qq[x], v, o);
+            if (col_ok && key + x < d) row[(size_t)(4 * i + x) * e] = v;
         }
     }
     red[256 + warp * 32 + lane] = o;
@@ -517,8 +539,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) linear_step_kernel(ScanArgs a) {
 template <int MODE>
 static int dispatch_step(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
     const dim3 grid(n_seqs, a.H, (a.e + 31) / 32);
-    const size_t smem = (SCAN_STEP_VECTORS(MODE) * (size_t)a.d + 384) * sizeof(float);
-#define TQ_STEP(K) return tq_launch_pdl(TQ_PDL_ELEMENTWISE, linear_step_kernel<MODE, K>, grid, dim3(SCAN_THREADS), smem, stream, a)
+#define TQ_STEP(K)                                                                                                       \
+    do {                                                                                                                 \
+        const size_t smem = (SCAN_STEP_VECTORS(MODE) * (size_t)(4 * K) + 384) * sizeof(float);                           \
+        return tq_launch_pdl(TQ_PDL_ELEMENTWISE, linear_step_kernel<MODE, K>, grid, dim3(SCAN_THREADS), smem, stream, a); \
+    } while (0)
     if (a.d <= 32) TQ_STEP(8);
     if (a.d <= 64) TQ_STEP(16);
     if (a.d <= 128) TQ_STEP(32);
