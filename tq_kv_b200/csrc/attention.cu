@@ -192,9 +192,10 @@ __global__ void attention_kernel(const TC* __restrict__ q, KVSource src, const i
 
 // Merges the splits of one (token, head): grid (token, head).  Bound by latency: a thread takes 16 bytes of the row and
 // every G-th split (G groups, about one for four splits), and asks for its first eight before it looks at the maxima, so
-// that up to 64 splits of a row of 128 arrive together (with the 128 threads of before, each walking all splits, 48 of them
-// took 10 us a layer; rirudra-2k, 24 tokens after a prompt of 3,000, 24 to 36 splits of 256: 8.70 -> 8.51 ms a pass); the groups meet in shared memory.  Splits are combined in a fixed order, so the
-// result does not depend on scheduling.  An empty split has m = -inf and l = 0 and contributes nothing.
+// that up to 64 splits of a row of 128 arrive together; the groups meet in shared memory.  (With the 128 threads of before,
+// each walking all splits, 48 of them took 10 us a layer; rirudra-2k, 24 tokens after a prompt of 3,000, 24 to 36 splits of
+// 256: 8.70 -> 8.51 ms a pass.)  Splits are combined in a fixed order, so the result does not depend on scheduling.  An
+// empty split has m = -inf and l = 0 and contributes nothing.
 #define AM_THREADS 256
 #define AM_AHEAD 8
 template <typename TC>
