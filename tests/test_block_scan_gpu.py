@@ -35,7 +35,7 @@ def make(mode, lens, H, G, d, e, seed):
     return p
 
 
-def exact(mode, p, lens, slots, H, G, d, e):
+def exact(mode, p, lens, slots, H, G, d, e, eps=1e-6):
     T = sum(lens)
     q, k, v = (p[n].double() for n in "qkv")
     if mode == "decay":
@@ -45,7 +45,7 @@ def exact(mode, p, lens, slots, H, G, d, e):
     out, state, t = torch.empty(T, H, e, dtype=torch.float64, device=DEV), p["state"].double().clone(), 0
     if mode == "delta":
         w = torch.exp(-math.exp(-0.5) * torch.sigmoid(p["w"].double())).reshape(T, H, d, 1)
-        u = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+        u = k / torch.sqrt((k * k).sum(-1, keepdim=True) + eps)
         na = -(torch.sigmoid(p["a"].double()).reshape(T, H, d) * u)
     for n, slot in zip(lens, slots):
         S = state[slot].reshape(H, d, e)
@@ -67,7 +67,7 @@ def exact(mode, p, lens, slots, H, G, d, e):
     return out.reshape(T, H * e), state
 
 
-def run(mode, p, lens, slots, H, G, d, e):
+def run(mode, p, lens, slots, H, G, d, e, eps=1e-6):
     from tq_kv_b200 import kernels
     T, cu = sum(lens), [0]
     for n in lens:
@@ -75,7 +75,7 @@ def run(mode, p, lens, slots, H, G, d, e):
     out, state = torch.full((T, H * e), float("nan"), device=DEV), p["state"].clone()
     if mode in ("delta", "decay"):
         cols = [p["q"], p["k"], p["v"]] + ([p["a"]] if mode == "delta" else [])
-        kw = dict(decay_logit=p["w"].clone(), off_a=2 * H * d + H * e) if mode == "delta" else dict(head_decay=p["c"], silu=True)
+        kw = dict(decay_logit=p["w"].clone(), off_a=2 * H * d + H * e, unit_eps=eps) if mode == "delta" else dict(head_decay=p["c"], silu=True)
         kernels.linear_scan(torch.cat(cols, 1), state.reshape(-1, H, d, e), i32(cu), i32(slots), out, n_seqs=len(lens), heads=H,
                             key_dim=d, value_dim=e, off_q=0, off_k=H * d, off_v=2 * H * d, **kw)
     else:
@@ -130,3 +130,14 @@ def test_a_token_changes_nothing_before_it(mode):
     p["v"][5] = float("inf")
     spoiled, _ = run(mode, p, lens, [0], H, H, d, d)
     assert torch.equal(out[:5], spoiled[:5]) and not torch.isfinite(spoiled[5]).any()
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 13])
+def test_a_unit_key_without_a_floor(n):
+    """unit_eps = 0: the tokens that fill a sequence's last eight have no key to divide by."""
+    lens, H, d = [n, 20], 2, 64
+    p = make("delta", lens, H, H, d, d, seed=n)
+    out, state = run("delta", p, lens, [1, 3], H, H, d, d, eps=0.0)
+    want, want_state = exact("delta", p, lens, [1, 3], H, H, d, d, eps=0.0)
+    for got, ref in ((out, want), (state, want_state)):
+        assert float((got.double() - ref).abs().max()) <= 2e-6 * float(ref.abs().max())

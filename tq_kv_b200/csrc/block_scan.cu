@@ -141,8 +141,8 @@ __global__ void block_prepare_kernel(ScanArgs a, int n_seqs, int rec0, float* re
         for (int j = 0; j < TK; ++j) {
             float sum = 0.f;
             for (int x = 0; x < dp / 32; ++x) sum += norm[x * TK + j];
-            b[j] = k[j] * (1.f / sqrtf(sum + a.unit_eps));
             const bool here = i < a.d && j < n;
+            b[j] = here ? k[j] * (1.f / sqrtf(sum + a.unit_eps)) : 0.f;   // (no token: no key to divide by, whatever unit_eps is)
             na[j] = here ? -(bs_sigmoid(na[j]) * b[j]) : 0.f;
             w[j] = here ? expf(-0.6065306597126334f * bs_sigmoid(w[j])) : 1.f;
         }
