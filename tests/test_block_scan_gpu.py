@@ -141,3 +141,18 @@ def test_a_unit_key_without_a_floor(n):
     want, want_state = exact("delta", p, lens, [1, 3], H, H, d, d, eps=0.0)
     for got, ref in ((out, want), (state, want_state)):
         assert float((got.double() - ref).abs().max()) <= 2e-6 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("mode", ["delta", "gated_delta"])
+def test_an_infinite_state_entry_meets_no_token_that_is_not_there(mode):
+    """One token: the other entries of the column become infinite with the sign that their key's removal gives, none NaN."""
+    H, d, lens = 2, 64, [1]
+    p = make(mode, lens, H, H, d, d, seed=2)
+    p["state"].reshape(-1, H, d, d)[1, 0, 5, 9] = float("inf")
+    out, state = run(mode, p, lens, [1], H, H, d, d)
+    want, want_state = exact(mode, p, lens, [1], H, H, d, d)
+    fine = torch.isfinite(want_state)
+    assert int((~fine).sum()) == d and int(torch.isnan(want_state).sum()) == 1
+    assert torch.equal(torch.isnan(state), torch.isnan(want_state))
+    assert torch.equal(state[~fine].nan_to_num(), want_state[~fine].float().nan_to_num())
+    assert float((state.double() - want_state)[fine].abs().max()) <= 2e-6 * float(want_state[fine].abs().max())

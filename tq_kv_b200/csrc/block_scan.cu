@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(THREADS) block_scan_kernel(ScanArgs a, int rec
         keep_v(i + 1);
         fetch_v(i + 2);
         if (i > 0) write_out(i - 1);
+        const int here = t1 - (tb + i * TK);              // tokens of this record (a count past TK is as good)
         const float* sc = sm + (i % BS_STAGES) * REC;
         const float4* pv = reinterpret_cast<const float4*>(sc) + kg;
         float val[V];
@@ -395,6 +396,7 @@ __global__ void __launch_bounds__(THREADS) block_scan_kernel(ScanArgs a, int rec
 #pragma unroll
             for (int j = 0; j < TK; ++j)
                 if (j < limit) sum = fmaf(m[j], u[j], sum);              // (a later token's value is not touched)
+            if (DELTA && row < TK && row >= here) sum = 0.f;             // (no token: 0, and not 0 * an infinite state)
             if (SAME == 1 || kg % SAME == 0) {
                 if (DELTA && row < TK) sr[(cg * RC + c) * BS_LDC + row] = sum;
                 else so[((i & 1) * TK + row - (DELTA ? TK : 0)) * CT + cg * RC + c] = sum;
