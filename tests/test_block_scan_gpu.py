@@ -156,3 +156,30 @@ def test_an_infinite_state_entry_meets_no_token_that_is_not_there(mode):
     assert torch.equal(torch.isnan(state), torch.isnan(want_state))
     assert torch.equal(state[~fine].nan_to_num(), want_state[~fine].float().nan_to_num())
     assert float((state.double() - want_state)[fine].abs().max()) <= 2e-6 * float(want_state[fine].abs().max())
+
+
+@pytest.mark.parametrize("d", [6, 40, 100, 200])
+@pytest.mark.parametrize("mode", MODES + ["channel_delta"])
+def test_one_token_with_an_infinite_value(mode, d):
+    """Key widths short of the kernel's: the keys that fill them up stay out of the sums (0 * inf is no 0)."""
+    from tq_kv_b200 import kernels
+    H, e = 2, d
+    g = torch.Generator(device=DEV).manual_seed(d)
+    pos = [torch.rand(1, H * d, generator=g, device=DEV) + 0.1 for _ in range(4)]       # q, k, v, removal logits
+    pos[2][0, 3] = float("inf")
+    state, out = torch.zeros(1, H, d, e, device=DEV), torch.empty(1, H * e, device=DEV)
+    cu, slots, buf, n = i32([0, 1]), i32([0]), torch.cat(pos, 1), H * d
+    scal = torch.full((1, H, 4), 0.5, device=DEV)
+    common = dict(n_seqs=1, heads=H, key_dim=d, value_dim=e, single_tokens=True)
+    qkv = (buf[:, :n], buf[:, n:2 * n], buf[:, 2 * n:3 * n])
+    if mode in ("delta", "decay"):
+        kw = (dict(decay_logit=torch.zeros(1, n, device=DEV), off_a=3 * n) if mode == "delta"
+              else dict(head_decay=torch.full((H,), 0.5, device=DEV)))
+        kernels.linear_scan(buf, state, cu, slots, out, off_q=0, off_k=n, off_v=2 * n, **common, **kw)
+    elif mode == "channel_delta":
+        kernels.channel_delta_scan(*qkv, torch.full((1, n), 0.5, device=DEV), scal, state.reshape(1, -1), cu, slots, out,
+                                   qk_heads=H, **common)
+    else:
+        kernels.gated_scan(*qkv, scal, state.reshape(1, -1), cu, slots, out, qk_heads=H, delta=mode == "gated_delta", **common)
+    assert float(out[0, 3]) == float("inf") and bool((state[0, 0, :, 3] == float("inf")).all())
+    assert bool(torch.isfinite(out[0, 4:]).all()) and bool(torch.isfinite(state[0, 0, :, 4:]).all())

@@ -523,8 +523,9 @@ __global__ void __launch_bounds__(SCAN_THREADS, KPW <= 32 ? SCAN_STEP_BLOCKS(MOD
             float v = S[4 * i + x];
             if (MODE == SCAN_DELTA) v = fmaf(ww[x], v, fmaf(kk[x], vj, aa[x] * dot));
             else v = fmaf(ww[x], v, kk[x] * vw);
+            if (key + x >= d) continue;                       // (no key: 0 * an infinite value is no 0)
             o = fmaf(qq[x], v, o);
-            if (col_ok && key + x < d) row[(size_t)(4 * i + x) * e] = v;
+            if (col_ok) row[(size_t)(4 * i + x) * e] = v;
         }
     }
     red[256 + warp * 32 + lane] = o;
