@@ -12,7 +12,7 @@ DEV = "cuda"
 
 
 def i32(x):
-    return torch.tensor(x, dtype=torch.int32, device=DEV)
+    return torch.tensor(list(x), dtype=torch.int32, device=DEV)
 
 
 def make(mode, lens, H, G, d, e, seed):
@@ -158,28 +158,57 @@ def test_an_infinite_state_entry_meets_no_token_that_is_not_there(mode):
     assert float((state.double() - want_state)[fine].abs().max()) <= 2e-6 * float(want_state[fine].abs().max())
 
 
-@pytest.mark.parametrize("d", [6, 40, 100, 200])
-@pytest.mark.parametrize("mode", MODES + ["channel_delta"])
-def test_one_token_with_an_infinite_value(mode, d):
-    """Key widths short of the kernel's: the keys that fill them up stay out of the sums (0 * inf is no 0)."""
+def one_token(mode, p, state, H, d):
+    """A token of each sequence through the kernel for one token; decays, steps and strengths of a half where not given."""
     from tq_kv_b200 import kernels
-    H, e = 2, d
-    g = torch.Generator(device=DEV).manual_seed(d)
-    pos = [torch.rand(1, H * d, generator=g, device=DEV) + 0.1 for _ in range(4)]       # q, k, v, removal logits
-    pos[2][0, 3] = float("inf")
-    state, out = torch.zeros(1, H, d, e, device=DEV), torch.empty(1, H * e, device=DEV)
-    cu, slots, buf, n = i32([0, 1]), i32([0]), torch.cat(pos, 1), H * d
-    scal = torch.full((1, H, 4), 0.5, device=DEV)
-    common = dict(n_seqs=1, heads=H, key_dim=d, value_dim=e, single_tokens=True)
+    T, n = p["q"].shape
+    buf, out, cu, slots = torch.cat([p[x] for x in "qkva"], 1), torch.empty(T, n, device=DEV), i32(range(T + 1)), i32(range(T))
+    scal = torch.full((T, H, 4), 0.5, device=DEV)
+    common = dict(n_seqs=T, heads=H, key_dim=d, value_dim=d, single_tokens=True)
     qkv = (buf[:, :n], buf[:, n:2 * n], buf[:, 2 * n:3 * n])
     if mode in ("delta", "decay"):
-        kw = (dict(decay_logit=torch.zeros(1, n, device=DEV), off_a=3 * n) if mode == "delta"
-              else dict(head_decay=torch.full((H,), 0.5, device=DEV)))
+        kw = dict(decay_logit=p["w"], off_a=3 * n) if mode == "delta" else dict(head_decay=torch.full((H,), 0.5, device=DEV))
         kernels.linear_scan(buf, state, cu, slots, out, off_q=0, off_k=n, off_v=2 * n, **common, **kw)
     elif mode == "channel_delta":
-        kernels.channel_delta_scan(*qkv, torch.full((1, n), 0.5, device=DEV), scal, state.reshape(1, -1), cu, slots, out,
-                                   qk_heads=H, **common)
+        kernels.channel_delta_scan(*qkv, torch.sigmoid(p["w"]), scal, state.reshape(T, -1), cu, slots, out, qk_heads=H, **common)
     else:
-        kernels.gated_scan(*qkv, scal, state.reshape(1, -1), cu, slots, out, qk_heads=H, delta=mode == "gated_delta", **common)
-    assert float(out[0, 3]) == float("inf") and bool((state[0, 0, :, 3] == float("inf")).all())
-    assert bool(torch.isfinite(out[0, 4:]).all()) and bool(torch.isfinite(state[0, 0, :, 4:]).all())
+        kernels.gated_scan(*qkv, scal, state.reshape(T, -1), cu, slots, out, qk_heads=H, delta=mode == "gated_delta", **common)
+    return state, out
+
+
+@pytest.mark.parametrize("d", [6, 40, 100, 200])
+@pytest.mark.parametrize("mode", MODES + ["channel_delta"])
+@pytest.mark.parametrize("n", [1, 320])
+def test_one_token_with_an_infinite_value(mode, d, n):
+    """Key widths short of the kernel's: the keys that fill them up stay out of the sums (0 * inf is no 0)."""
+    H, g = 2, torch.Generator(device=DEV).manual_seed(d)
+    p = {x: torch.rand(n, H * d, generator=g, device=DEV) + 0.1 for x in "qkvaw"}
+    p["v"][-1, 3] = float("inf")
+    state, out = one_token(mode, p, torch.zeros(n, H, d, d, device=DEV), H, d)
+    assert float(out[-1, 3]) == float("inf") and bool((state[-1, 0, :, 3] == float("inf")).all())
+    assert int((~torch.isfinite(out)).sum()) == 1 and int((~torch.isfinite(state)).sum()) == d
+
+
+@pytest.mark.parametrize("d,H,n", [(32, 2, 1), (32, 4, 200), (64, 2, 3), (64, 4, 80), (128, 2, 3), (128, 16, 8), (128, 8, 40), (256, 2, 2),
+                                   (256, 4, 20), (6, 2, 2), (6, 4, 170), (40, 2, 2), (40, 4, 100), (100, 2, 2), (100, 8, 40), (200, 1, 3),
+                                   (200, 4, 30)])
+@pytest.mark.parametrize("mode", MODES + ["channel_delta"])
+def test_one_token_against_float64(mode, d, H, n):
+    """Whole and other widths, from a few blocks to more than four an SM."""
+    g = torch.Generator(device=DEV).manual_seed(d + n)
+    p = {x: torch.randn(n, H * d, generator=g, device=DEV) for x in "qkvaw"}
+    p["k"] = torch.nn.functional.normalize(p["k"].reshape(n, H, d), dim=-1).reshape(n, -1)
+    before = torch.randn(n, H, d, d, generator=g, device=DEV)
+    state, out = one_token(mode, p, before.clone(), H, d)
+    q, k, v, a, w = (p[x].double().reshape(n, H, d) for x in "qkvaw")
+    S = before.double()
+    if mode == "delta":
+        w, u = torch.exp(-math.exp(-0.5) * torch.sigmoid(w)), k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+        S = w[..., None] * S - (torch.sigmoid(a) * u)[..., None] * (u[:, :, None] @ S) + k[..., None] * v[:, :, None]
+    else:
+        S = S * (torch.sigmoid(w)[..., None] if mode == "channel_delta" else 0.5)
+        x = v if mode == "decay" else 0.5 * (v - (k[:, :, None] @ S)[:, :, 0] if "delta" in mode else v)
+        S = S + k[..., None] * x[:, :, None]
+    want = (q[:, :, None] @ S)[:, :, 0].reshape(n, -1)
+    for got, ref in ((out, want), (state, S)):
+        assert float((got.double() - ref).abs().max()) <= 2e-6 * float(ref.abs().max())

@@ -410,24 +410,28 @@ static int dispatch_scan(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
 }
 
 // ---------------------------------------------------------------------------
-// linear_step: one token per sequence.  Warp w of a block owns a quarter of the keys and 32 columns; partial dot
-// products meet in shared memory.  The token's vectors are staged once per block and read four keys at a time.
+// linear_step: one token per sequence.  A warp owns a quarter of the keys and the block 32 columns; partial dot products
+// meet in shared memory.  The token's vectors are staged once per block.  Bound by how much of the state is on its way.
+// Three forms (which one: dispatch_step):
+//   STEP_WHOLE    a warp owns KPW neighbouring keys and reads the vectors four keys at a time; widths d = 4 * KPW, so that no
+//                 key needs a look whether it is there (those looks cost up to a quarter of the time)
+//   STEP_PART     the same for d < 4 * KPW
+//   STEP_EVERY4   a warp owns every fourth key and reads the vectors one by one, d <= 4 * KPW
 // ---------------------------------------------------------------------------
+#define STEP_WHOLE 0
+#define STEP_PART 1
+#define STEP_EVERY4 2
 #define SCAN_STEP_VECTORS(MODE) ((MODE) == SCAN_DELTA ? 5 : ((MODE) == SCAN_CHANNEL_DELTA ? 4 : 2))
-// Blocks an SM, by rule: as many as leave the state's registers unspilled.  Measured in replayed graphs, 64 sequences, 16
-// heads of 128 x 128 (134 MB read and written), in us, four blocks of 128 registers and one key a load before / now: delta
-// rule 39.6 / 35.7, constant decay 34.2 / 28.2, one decay with the delta rule 42.0 / 31.8 (floor 20.5).
-#define SCAN_STEP_BLOCKS(MODE) ((MODE) == SCAN_DECAY ? 8 : ((MODE) == SCAN_GATED_DELTA ? 6 : ((MODE) == SCAN_DELTA ? 5 : 4)))
-template <int MODE, int KPW>      // KPW: keys per warp (d <= 4 * KPW)
-__global__ void __launch_bounds__(SCAN_THREADS, KPW <= 32 ? SCAN_STEP_BLOCKS(MODE) : 1) linear_step_kernel(ScanArgs a) {
-    constexpr int DP = 4 * KPW;                               // the vectors' keys from d on are zeros
+template <int MODE, int KPW, int FORM, int BLOCKS>      // BLOCKS: that share an SM, at least (0: the compiler's choice)
+__global__ void __launch_bounds__(SCAN_THREADS, BLOCKS) linear_step_kernel(ScanArgs a) {
+    constexpr int DP = 4 * KPW;                               // STEP_PART: the vectors' entries from d on are zeros
     extern __shared__ __align__(16) float sm[];
     const int b = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
     const int d = a.d, e = a.e, col = col0 + lane;
     const int hq = head / a.qk_div;
     const bool col_ok = col < e;
-    float* sq = sm;                 // [d] each: q k (u au w; or the products w k in u's place, then w)
+    float* sq = sm;                 // [DP] each: q k (u au w; or the products w k in u's place, then w)
     float* sk = sq + DP;
     float* su = sk + DP;
     float* sau = su + DP;
@@ -441,13 +445,13 @@ __global__ void __launch_bounds__(SCAN_THREADS, KPW <= 32 ? SCAN_STEP_BLOCKS(MOD
     float S[KPW];
 #pragma unroll
     for (int i = 0; i < KPW; ++i) {
-        const int key = warp * KPW + i;
-        S[i] = (col_ok && key < d) ? st[(size_t)key * e + col] : 0.f;
+        const int key = FORM == STEP_EVERY4 ? i * 4 + warp : warp * KPW + i;
+        S[i] = (col_ok && (FORM == STEP_WHOLE || key < d)) ? st[(size_t)key * e + col] : 0.f;
     }
     // the token's vectors, made here from the projections' results (one token: no prepare kernel runs before)
     float ss = 0.f;
-    for (int i = tid; i < DP; i += SCAN_THREADS) {
-        if (i >= d) {
+    for (int i = tid; i < (FORM == STEP_PART ? DP : d); i += SCAN_THREADS) {
+        if (FORM == STEP_PART && i >= d) {
             sq[i] = sk[i] = 0.f;
             if (MODE == SCAN_DELTA) su[i] = sau[i] = sw[i] = 0.f;
             if (MODE == SCAN_CHANNEL_DELTA) su[i] = sw[i] = 0.f;
@@ -489,14 +493,22 @@ __global__ void __launch_bounds__(SCAN_THREADS, KPW <= 32 ? SCAN_STEP_BLOCKS(MOD
         s2 = a.scal[((size_t)t * a.H + head) * 4 + 1];
     }
     if (MODE == SCAN_DELTA || MODE == SCAN_GATED_DELTA || MODE == SCAN_CHANNEL_DELTA) {
-        const float4* sd = reinterpret_cast<const float4*>((MODE == SCAN_GATED_DELTA ? sk : su) + warp * KPW);
+        const float* sd = MODE == SCAN_GATED_DELTA ? sk : su;
+        if constexpr (FORM == STEP_EVERY4) {
 #pragma unroll
-        for (int i = 0; i < KPW / 4; ++i) {
-            const float4 x = sd[i];
-            dot = fmaf(x.x, S[4 * i], dot);
-            dot = fmaf(x.y, S[4 * i + 1], dot);
-            dot = fmaf(x.z, S[4 * i + 2], dot);
-            dot = fmaf(x.w, S[4 * i + 3], dot);
+            for (int i = 0; i < KPW; ++i) {
+                const int key = i * 4 + warp;
+                if (key < d) dot = fmaf(sd[key], S[i], dot);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < KPW / 4; ++i) {
+                const float4 x = reinterpret_cast<const float4*>(sd + warp * KPW)[i];
+                dot = fmaf(x.x, S[4 * i], dot);
+                dot = fmaf(x.y, S[4 * i + 1], dot);
+                dot = fmaf(x.z, S[4 * i + 2], dot);
+                dot = fmaf(x.w, S[4 * i + 3], dot);
+            }
         }
         red[128 + warp * 32 + lane] = dot;
         __syncthreads();
@@ -508,24 +520,38 @@ __global__ void __launch_bounds__(SCAN_THREADS, KPW <= 32 ? SCAN_STEP_BLOCKS(MOD
     if (MODE == SCAN_GATED) vw = s2 * vj;
     if (MODE == SCAN_GATED_DELTA) vw = s2 * (vj - g * dot);
     if (MODE == SCAN_CHANNEL_DELTA) vw = s2 * (vj - dot);
-    float* row = st + (size_t)warp * KPW * e + col;
+    if constexpr (FORM == STEP_EVERY4) {
 #pragma unroll
-    for (int i = 0; i < KPW / 4; ++i) {
-        const int key = warp * KPW + 4 * i;
-        const float4 k4 = *reinterpret_cast<const float4*>(sk + key), q4 = *reinterpret_cast<const float4*>(sq + key);
-        float4 w4 = make_float4(c_head, c_head, c_head, c_head), a4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (MODE == SCAN_DELTA || MODE == SCAN_CHANNEL_DELTA) w4 = *reinterpret_cast<const float4*>(sw + key);
-        if (MODE == SCAN_DELTA) a4 = *reinterpret_cast<const float4*>(sau + key);
-        const float kk[4] = {k4.x, k4.y, k4.z, k4.w}, qq[4] = {q4.x, q4.y, q4.z, q4.w}, ww[4] = {w4.x, w4.y, w4.z, w4.w},
-                    aa[4] = {a4.x, a4.y, a4.z, a4.w};
+        for (int i = 0; i < KPW; ++i) {
+            const int key = i * 4 + warp;
+            if (key < d) {
+                if (MODE == SCAN_DELTA) S[i] = fmaf(sw[key], S[i], fmaf(sk[key], vj, sau[key] * dot));
+                else if (MODE == SCAN_CHANNEL_DELTA) S[i] = fmaf(sw[key], S[i], sk[key] * vw);
+                else S[i] = fmaf(c_head, S[i], sk[key] * vw);
+                o = fmaf(sq[key], S[i], o);
+                if (col_ok) st[(size_t)key * e + col] = S[i];
+            }
+        }
+    } else {
+        float* row = st + (size_t)warp * KPW * e + col;
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            float v = S[4 * i + x];
-            if (MODE == SCAN_DELTA) v = fmaf(ww[x], v, fmaf(kk[x], vj, aa[x] * dot));
-            else v = fmaf(ww[x], v, kk[x] * vw);
-            if (key + x >= d) continue;                       // (no key: 0 * an infinite value is no 0)
-            o = fmaf(qq[x], v, o);
-            if (col_ok) row[(size_t)(4 * i + x) * e] = v;
+        for (int i = 0; i < KPW / 4; ++i) {
+            const int key = warp * KPW + 4 * i;
+            const float4 k4 = *reinterpret_cast<const float4*>(sk + key), q4 = *reinterpret_cast<const float4*>(sq + key);
+            float4 w4 = make_float4(c_head, c_head, c_head, c_head), a4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (MODE == SCAN_DELTA || MODE == SCAN_CHANNEL_DELTA) w4 = *reinterpret_cast<const float4*>(sw + key);
+            if (MODE == SCAN_DELTA) a4 = *reinterpret_cast<const float4*>(sau + key);
+            const float kk[4] = {k4.x, k4.y, k4.z, k4.w}, qq[4] = {q4.x, q4.y, q4.z, q4.w}, ww[4] = {w4.x, w4.y, w4.z, w4.w},
+                        aa[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                float v = S[4 * i + x];
+                if (MODE == SCAN_DELTA) v = fmaf(ww[x], v, fmaf(kk[x], vj, aa[x] * dot));
+                else v = fmaf(ww[x], v, kk[x] * vw);
+                if (FORM == STEP_PART && key + x >= d) continue;              // (no key: 0 * an infinite value is no 0)
+                o = fmaf(qq[x], v, o);
+                if (col_ok) row[(size_t)(4 * i + x) * e] = v;
+            }
         }
     }
     red[256 + warp * 32 + lane] = o;
@@ -537,18 +563,44 @@ __global__ void __launch_bounds__(SCAN_THREADS, KPW <= 32 ? SCAN_STEP_BLOCKS(MOD
     }
 }
 
+// Which form, and how many blocks an SM (as many as leave the registers unspilled).  Measured in replayed graphs, 128 x 128
+// states of 16 heads, in us, every fourth key / whole:
+//                 1 sequence   8             32             64 (floor 20.5)
+//   delta rule    3.86 / 3.46  6.94 / 7.18   22.3 / 18.9    39.7 / 34.9
+//   constant      3.36 / 3.18  6.01 / 6.18   19.2 / 15.6    34.4 / 28.4
+//   gated         3.20 / 2.89  5.99 / 6.29   18.9 / 16.8    34.1 / 30.5
+//   gated delta   3.52 / 2.88  8.82 / 6.83   23.5 / 16.8    42.5 / 29.2
+//   channel delta 3.25 / 2.91  8.13 / 5.96   21.9 / 19.1    39.3 / 34.0
+// so whole widths take the whole form, but for the gated rule while there are more blocks than SMs and four an SM take them
+// all (the 512 of 8 sequences; of 4: 4.64 / 5.48 with looks).  64 sequences at 64 x 64: 13.8 / 12.4, 9.7 / 9.6, 9.7 / 9.2,
+// 11.7 / 9.3, 11.2 / 9.4; at 32 x 32: 4.7 / 4.2, 4.1 / 3.9, 3.8 / 3.7, 3.9 / 3.7, 3.8 / 3.8; 32 sequences at 256 x 256: 131
+// / 90, 100 / 79, 99 / 77, 108 / 77, 108 / 80.  Other widths, 100 x 100, every fourth / part: delta 1 sequence 3.9 / 3.8, 8 5.6 /
+// 6.0, 64 35.7 / 33.9; constant 3.5 / 3.7, 4.7 / 5.1, 29.4 / 26.7; gated 3.1 / 4.2, 4.4 / 5.7, 28.5 / 36.3; gated delta 3.3 /
+// 3.5, 7.2 / 5.9, 37.2 / 27.5; channel delta 3.4 / 3.6, 7.5 / 5.2, 38.1 / 33.5.
 template <int MODE>
 static int dispatch_step(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
     const dim3 grid(n_seqs, a.H, (a.e + 31) / 32);
-#define TQ_STEP(K)                                                                                                       \
-    do {                                                                                                                 \
-        const size_t smem = (SCAN_STEP_VECTORS(MODE) * (size_t)(4 * K) + 384) * sizeof(float);                           \
-        return tq_launch_pdl(TQ_PDL_ELEMENTWISE, linear_step_kernel<MODE, K>, grid, dim3(SCAN_THREADS), smem, stream, a); \
+    const long long blocks = (long long)n_seqs * a.H * grid.z, sms = tq_sm_count();
+    constexpr int BLOCKS = MODE == SCAN_DECAY ? 7 : (MODE == SCAN_GATED_DELTA ? 6 : (MODE == SCAN_DELTA ? 5 : 4));
+#define TQ_STEP(K, FORM, BLOCKS)                                                                                      \
+    do {                                                                                                              \
+        const size_t smem = (SCAN_STEP_VECTORS(MODE) * (size_t)(4 * K) + 384) * sizeof(float);                        \
+        return tq_launch_pdl(TQ_PDL_ELEMENTWISE, linear_step_kernel<MODE, K, FORM, BLOCKS>, grid, dim3(SCAN_THREADS), \
+                             smem, stream, a);                                                                        \
     } while (0)
-    if (a.d <= 32) TQ_STEP(8);
-    if (a.d <= 64) TQ_STEP(16);
-    if (a.d <= 128) TQ_STEP(32);
-    TQ_STEP(64);
+#define TQ_STEP_WIDTHS(K, BLOCKS)                                                                               \
+    do {                                                                                                        \
+        if (a.d == 4 * K && !every4) TQ_STEP(K, STEP_WHOLE, BLOCKS);                                            \
+        if constexpr (MODE != SCAN_GATED)                                                                       \
+            if (blocks > (MODE == SCAN_DELTA || MODE == SCAN_DECAY ? 4 : 1) * sms) TQ_STEP(K, STEP_PART, BLOCKS); \
+        TQ_STEP(K, STEP_EVERY4, (MODE == SCAN_DELTA && K == 32 ? 4 : 0));                                       \
+    } while (0)
+    const bool every4 = MODE == SCAN_GATED && a.d == 128 && blocks > sms && blocks <= 4 * sms;
+    if (a.d <= 32) TQ_STEP_WIDTHS(8, BLOCKS);
+    if (a.d <= 64) TQ_STEP_WIDTHS(16, (MODE == SCAN_GATED_DELTA ? 7 : BLOCKS));
+    if (a.d <= 128) TQ_STEP_WIDTHS(32, BLOCKS);
+    TQ_STEP_WIDTHS(64, 1);
+#undef TQ_STEP_WIDTHS
 #undef TQ_STEP
 }
 
