@@ -212,3 +212,23 @@ def test_one_token_against_float64(mode, d, H, n):
     want = (q[:, :, None] @ S)[:, :, 0].reshape(n, -1)
     for got, ref in ((out, want), (state, S)):
         assert float((got.double() - ref).abs().max()) <= 2e-6 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_no_less_exact_than_token_by_token(mode, monkeypatch):
+    """The errors of both kernels against float64, in the norm.  Slow constant decays are the hardest: a rounding of their
+    product over eight tokens is the same for each record and adds up over all that the state remembers."""
+    from tq_kv_b200.kernels import scan
+    lens, H, d = [803], 2, 128
+    p = make(mode, lens, H, H, d, d, seed=7)
+    if mode == "decay":
+        p["c"] = torch.tensor([0.9, 0.996], device=DEV)
+    want, want_state = exact(mode, p, lens, [0], H, H, d, d)
+    errors = []
+    for records in (scan._records, lambda *a: None):
+        monkeypatch.setattr(scan, "_records", records)
+        out, state = run(mode, p, lens, [0], H, H, d, d)
+        errors.append([float((out.double() - want).norm() / want.norm()),
+                       float((state[0].double() - want_state[0]).norm() / want_state[0].norm())])
+    eight, one = errors
+    assert eight[0] <= 1.1 * one[0] and eight[1] <= 1.1 * one[1], errors

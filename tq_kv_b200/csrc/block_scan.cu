@@ -30,11 +30,18 @@
 //                 (cp.async).  The sums over the KG lanes that share a column are made by trading halves of the values,
 //                 so that each lane ends with the few sums that it completes (F v, E v) and hands on.
 //
+// Rounding.  Eight tokens' decays are one factor here, and a rounding of it that is the same for every record (a constant
+// decay) would not average out over the tokens that a slow decay remembers: the factor is kept as hi + lo, and so are the
+// products of decays that go into the vectors; the Gram sums are compensated.  But for the delta rule with a decay per
+// channel the eight changes of the state are summed before they meet it.  Error of results / states against 64 bits, in
+// 1e-7 of their norm, 1,200 tokens of 4 heads of 128 x 128, token by token -> here (without these): delta rule 0.99 / 0.68 ->
+// 0.99 / 0.66 (1.34 / 0.71), one decay per token 1.02 / 0.76 -> 0.95 / 0.69 (1.28 / 0.94), with the delta rule 1.05 / 0.79
+// -> 1.03 / 0.70 (1.38 / 1.04), constant decays of 0.875 to 0.996 0.82 / 2.78 -> 0.74 / 1.04 (6.44 / 7.63).
+//
 // What bounds it: the latency from one record to the next (the exchange over the lanes, the completed sums through shared
 // memory and back: about 1.3 us, of which the 32 vectors' loads and products fill half).  Measured (one sequence of 3,000
-// tokens, 16 heads of 128 x 128, launches included; before, token by token): delta rule 1,083 -> 572 us, one decay per token
-// 719 -> 337, with the delta rule 900 -> 520, constant decay 709 -> 359; error of the results against 64 bits 1.0e-7 ->
-// 1.3e-7 of their norm, of the states 0.7e-7 in both.  A long step is cut into pieces of records that stay in the L2
+// tokens, 16 heads of 128 x 128, launches included; before, token by token): delta rule 1,081 -> 600 us, one decay per token
+// 718 -> 350, with the delta rule 899 -> 528, constant decay 708 -> 380.  A long step is cut into pieces of records that stay in the L2
 // (SCAN_PIECE_BYTES): the state waits in its slot between them.
 #include "common.cuh"
 #include "scan_modes.cuh"
@@ -45,13 +52,26 @@
 #define SCAN_PIECE_BYTES (96LL << 20)
 
 __host__ __device__ constexpr int bs_record(int dp, bool delta) {
-    return (delta ? 4 : 2) * BS_TOKENS * dp + dp + (delta ? 16 : 8) * BS_TOKENS;
+    return (delta ? 4 : 2) * BS_TOKENS * dp + 2 * dp + (delta ? 16 : 8) * BS_TOKENS;
 }
 // the first record of sequence b, whose first token is t0: leaves room for every sequence's part-filled last record
 __device__ __forceinline__ int bs_first_record(int t0, int b) { return (t0 + (BS_TOKENS - 1) * b) / BS_TOKENS; }
 
 __device__ __forceinline__ float bs_sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float bs_silu(float z) { return z / (1.f + expf(-z)); }
+
+// Sums and products kept as a float32 number and what its rounding left: hi + lo.
+__device__ __forceinline__ float2 bs_minus(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ void bs_add(float2& hi, float2& lo, float2 x) {
+    const float2 sum = __fadd2_rn(hi, x), part = bs_minus(sum, hi);
+    lo = __fadd2_rn(lo, __fadd2_rn(bs_minus(hi, bs_minus(sum, part)), bs_minus(x, part)));
+    hi = sum;
+}
+__device__ __forceinline__ void bs_times(float& hi, float& lo, float w) {
+    const float product = __fmul_rn(hi, w);
+    lo = fmaf(lo, w, fmaf(hi, w, -product));
+    hi = product;
+}
 
 // Sums V values over N lanes (powers of two; `l`: the lane's place among them) by trading halves: afterwards a lane
 // holds the full sums of values l * (V / N) .. in v[0 ..] (N > V: of value l / (N / V)).
@@ -169,14 +189,25 @@ __global__ void block_prepare_kernel(ScanArgs a, int n_seqs, int rec0, float* re
     for (int p = i; p < LEFT * RIGHT; p += dp) {
         const float4* x = reinterpret_cast<const float4*>(lf + (p / RIGHT) * ld);
         const float4* y = reinterpret_cast<const float4*>(rt + (p % RIGHT) * ld);
-        float2 s0 = make_float2(0.f, 0.f), s1 = s0;
-#pragma unroll 8
-        for (int c = 0; c < dp / 4; ++c) {
-            const float4 u = x[c], v = y[c];
-            s0 = __ffma2_rn(make_float2(u.x, u.y), make_float2(v.x, v.y), s0);
-            s1 = __ffma2_rn(make_float2(u.z, u.w), make_float2(v.z, v.w), s1);
+        float2 s0 = make_float2(0.f, 0.f), s1 = s0, l0 = s0, l1 = s0;
+#pragma unroll 2
+        for (int c = 0; c < dp / 4; c += 4) {
+            float4 u = x[c], v = y[c];
+            float2 a0 = __fmul2_rn(make_float2(u.x, u.y), make_float2(v.x, v.y));
+            float2 a1 = __fmul2_rn(make_float2(u.z, u.w), make_float2(v.z, v.w));
+#pragma unroll
+            for (int i = 1; i < 4; ++i) {
+                u = x[c + i]; v = y[c + i];
+                a0 = __ffma2_rn(make_float2(u.x, u.y), make_float2(v.x, v.y), a0);
+                a1 = __ffma2_rn(make_float2(u.z, u.w), make_float2(v.z, v.w), a1);
+            }
+            bs_add(s0, l0, a0);
+            bs_add(s1, l1, a1);
         }
-        gram[p] = (s0.x + s1.x) + (s0.y + s1.y);
+        bs_add(s0, l0, s1);
+        float2 t = make_float2(s0.x, 0.f), lo = make_float2((l0.x + l1.x) + (l0.y + l1.y), 0.f);
+        bs_add(t, lo, make_float2(s0.y, 0.f));
+        gram[p] = t.x + lo.x;
     }
     __syncthreads();
     // A, B, C, D: what token p's reading (A, B) or query (C, D) meets of token s's removal and write
@@ -206,7 +237,7 @@ __global__ void block_prepare_kernel(ScanArgs a, int n_seqs, int rec0, float* re
 
     // the rows of F (r) and E (o): the last warp's lane j makes column j
     if (warp == dp / 32 - 1 && lane < TK) {
-        float* rows = out + (DELTA ? 4 : 2) * TK * dp + dp;
+        float* rows = out + (DELTA ? 4 : 2) * TK * dp + 2 * dp;
         const int j = lane;
         float f[TK];
         if (DELTA) {
@@ -234,44 +265,44 @@ __global__ void block_prepare_kernel(ScanArgs a, int n_seqs, int rec0, float* re
         }
     }
 
-    // the vectors: P, Q | N, X | the decays' product
+    // the vectors: P, Q | N, X | the decays' product, and what its rounding left
     float* vq = out + (DELTA ? TK * dp : 0);
     float* vn = vq + TK * dp;
     float* vx = vn + (DELTA ? TK * dp : 0);
-    float run = 1.f, p[TK];
+    float run = 1.f, run_lo = 0.f, p[TK];
 #pragma unroll
     for (int j = 0; j < TK; ++j) {
         const float wj = MODE == SCAN_DELTA ? w[j] : (MODE == SCAN_DECAY ? (j < n ? a.head_decay[h] : 1.f) : sc[2 * j]);
         w[j] = wj;
         if (DELTA) {
-            float v = run * (MODE == SCAN_DELTA ? b[j] : k[j]);
+            const float read = MODE == SCAN_DELTA ? b[j] : k[j];
+            float v = fmaf(run, read, run_lo * read);
 #pragma unroll
             for (int m = 0; m < j; ++m) v = fmaf(A[j * TK + m], p[m], v);
             p[j] = v;
             out[j * dp + i] = v;
         }
-        run *= wj;
-        float y = run * q[j];
+        bs_times(run, run_lo, wj);
+        float y = fmaf(run, q[j], run_lo * q[j]);
         if (DELTA) {
 #pragma unroll
             for (int m = 0; m <= j; ++m) y = fmaf(C[j * TK + m], p[m], y);
         }
         vq[j * dp + i] = y;
     }
-    float tail = 1.f;
+    float tail = 1.f, tail_lo = 0.f;
 #pragma unroll
     for (int j = TK - 1; j >= 0; --j) {
-        if (MODE == SCAN_DELTA) {
-            vn[j * dp + i] = tail * na[j];
-            vx[j * dp + i] = tail * k[j];
-        } else {
-            const float write = MODE == SCAN_DECAY ? 1.f : sc[2 * j + 1];
-            if (DELTA) vn[j * dp + i] = tail * (-(write * sc[2 * j]) * k[j]);
-            vx[j * dp + i] = tail * (write * k[j]);
-        }
-        tail *= w[j];
+        float x = k[j], y = MODE == SCAN_DELTA ? na[j] : 0.f;
+        if (MODE >= SCAN_GATED) x = sc[2 * j + 1] * k[j];
+        if (MODE == SCAN_GATED_DELTA) y = -(sc[2 * j + 1] * sc[2 * j]) * k[j];
+        if (DELTA) vn[j * dp + i] = fmaf(tail, y, tail_lo * y);
+        vx[j * dp + i] = fmaf(tail, x, tail_lo * x);
+        bs_times(tail, tail_lo, w[j]);
     }
-    vx[TK * dp + i] = run;
+    const float fade = run + run_lo;
+    vx[TK * dp + i] = fade;
+    vx[(TK + 1) * dp + i] = (run - fade) + run_lo;
 }
 
 __device__ __forceinline__ void bs_copy16(float* dst, const float* src) {
@@ -279,7 +310,8 @@ __device__ __forceinline__ void bs_copy16(float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
 
-template <bool DELTA, int KG, int RK, int THREADS, int RC>
+// APART: the eight tokens' changes of the state are summed before they meet it.
+template <bool DELTA, bool APART, int KG, int RK, int THREADS, int RC>
 __global__ void __launch_bounds__(THREADS) block_scan_kernel(ScanArgs a, int rec0, int rec1, int silu_v, const float* rec) {
     constexpr int TK = BS_TOKENS, DP = KG * RK, R4 = RK / 4, CT = THREADS / KG * RC, REC = bs_record(DP, DELTA);
     constexpr int ROWS = DELTA ? 16 : 8;                  // products with the state: r and o, or o
@@ -381,7 +413,7 @@ __global__ void __launch_bounds__(THREADS) block_scan_kernel(ScanArgs a, int rec
         }
         bs_trade_sums<KG, V>(val, kg);
         // this lane's sums get what the tokens before them in the record add
-        const float* rows = sc + (DELTA ? 4 : 2) * TK * DP + DP;
+        const float* rows = sc + (DELTA ? 4 : 2) * TK * DP + 2 * DP;
         const float* vcol = sv + ((i & 1) * CT + cg * RC) * BS_LDC;
 #pragma unroll
         for (int x = 0; x < PER; ++x) {
@@ -403,13 +435,19 @@ __global__ void __launch_bounds__(THREADS) block_scan_kernel(ScanArgs a, int rec
             }
         }
         __syncwarp();
+        float2 change[2 * R4][RC];
+        const float4* pf = pv + (DELTA ? 4 : 2) * TK * (DP / 4);
 #pragma unroll
         for (int g = 0; g < R4; ++g) {
-            const float4 fade = pv[(DELTA ? 4 : 2) * TK * (DP / 4) + g * KG];
+            const float4 hi = pf[g * KG], lo = pf[DP / 4 + g * KG];
 #pragma unroll
             for (int c = 0; c < RC; ++c) {
-                S[2 * g][c] = __fmul2_rn(make_float2(fade.x, fade.y), S[2 * g][c]);
-                S[2 * g + 1][c] = __fmul2_rn(make_float2(fade.z, fade.w), S[2 * g + 1][c]);
+                change[2 * g][c] = __fmul2_rn(make_float2(lo.x, lo.y), S[2 * g][c]);
+                change[2 * g + 1][c] = __fmul2_rn(make_float2(lo.z, lo.w), S[2 * g + 1][c]);
+                if (!APART) {
+                    change[2 * g][c] = __ffma2_rn(make_float2(hi.x, hi.y), S[2 * g][c], change[2 * g][c]);
+                    change[2 * g + 1][c] = __ffma2_rn(make_float2(hi.z, hi.w), S[2 * g + 1][c], change[2 * g + 1][c]);
+                }
             }
         }
 #pragma unroll
@@ -432,11 +470,21 @@ __global__ void __launch_bounds__(THREADS) block_scan_kernel(ScanArgs a, int rec
                         const float2 zz = make_float2(z, z);
 #pragma unroll
                         for (int g = 0; g < R4; ++g) {
-                            S[2 * g][c] = __ffma2_rn(make_float2(x[g].x, x[g].y), zz, S[2 * g][c]);
-                            S[2 * g + 1][c] = __ffma2_rn(make_float2(x[g].z, x[g].w), zz, S[2 * g + 1][c]);
+                            change[2 * g][c] = __ffma2_rn(make_float2(x[g].x, x[g].y), zz, change[2 * g][c]);
+                            change[2 * g + 1][c] = __ffma2_rn(make_float2(x[g].z, x[g].w), zz, change[2 * g + 1][c]);
                         }
                     }
                 }
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < R4; ++g) {
+            const float4 hi = APART ? pf[g * KG] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < RC; ++c) {
+                S[2 * g][c] = APART ? __ffma2_rn(make_float2(hi.x, hi.y), S[2 * g][c], change[2 * g][c]) : change[2 * g][c];
+                S[2 * g + 1][c] = APART ? __ffma2_rn(make_float2(hi.z, hi.w), S[2 * g + 1][c], change[2 * g + 1][c])
+                                        : change[2 * g + 1][c];
             }
         }
     }
@@ -454,7 +502,7 @@ __global__ void __launch_bounds__(THREADS) block_scan_kernel(ScanArgs a, int rec
 #define BS_SMEM_ALONE (116 * 1024)        // two such blocks do not fit the 228 KB of an SM
 #define BS_SMEM_PAIR (78 * 1024)          // three do not
 
-template <bool DELTA, int KG, int RK, int THREADS, int RC>
+template <bool DELTA, bool APART, int KG, int RK, int THREADS, int RC>
 static int launch_block_scan(const ScanArgs& a, int n_seqs, int rec0, int rec1, int silu_v, const float* rec, cudaStream_t stream) {
     constexpr int CT = THREADS / KG * RC, REC = bs_record(KG * RK, DELTA);
     size_t smem = ((size_t)BS_STAGES * REC + 3 * CT * BS_LDC + 2 * BS_TOKENS * CT) * sizeof(float);
@@ -464,7 +512,7 @@ static int launch_block_scan(const ScanArgs& a, int n_seqs, int rec0, int rec1, 
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(block_scan_kernel<DELTA, KG, RK, THREADS, RC>,
+        cudaError_t e = cudaFuncSetAttribute(block_scan_kernel<DELTA, APART, KG, RK, THREADS, RC>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
         if (e != cudaSuccess) return (int)e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
@@ -475,7 +523,7 @@ static int launch_block_scan(const ScanArgs& a, int n_seqs, int rec0, int rec1, 
     const long long blocks = (long long)grid.x * grid.y * grid.z;
     const size_t least = blocks <= tq_sm_count() ? BS_SMEM_ALONE : (blocks <= 2LL * tq_sm_count() ? BS_SMEM_PAIR : 0);
     if (smem < least) smem = least;
-    return tq_launch_pdl(TQ_PDL_ELEMENTWISE, block_scan_kernel<DELTA, KG, RK, THREADS, RC>, grid, dim3(THREADS), smem, stream, a, rec0,
+    return tq_launch_pdl(TQ_PDL_ELEMENTWISE, block_scan_kernel<DELTA, APART, KG, RK, THREADS, RC>, grid, dim3(THREADS), smem, stream, a, rec0,
                          rec1, silu_v, rec);
 }
 
@@ -483,10 +531,10 @@ static int launch_block_scan(const ScanArgs& a, int n_seqs, int rec0, int rec1, 
 // lanes; 8 or 16 columns a block.  Measured with 128 x 128 states, 3,000 tokens of one sequence, in us (columns a block x
 // threads; delta rule / one decay): 16 heads: 8 x 128 488 / 331, 16 x 256 490 / 346, 16 x 128 (eight keys a thread) 540 /
 // 352; 32 heads: 8 x 128 763 / 487, 16 x 128 702 / 568, 32 x 256 707 / 447.
-template <bool DELTA, int DP>
+template <bool DELTA, bool APART, int DP>
 static int pick_block_scan(const ScanArgs& a, int n_seqs, int rec0, int rec1, int silu_v, const float* rec, cudaStream_t stream) {
     constexpr int KG = DP >= 128 ? 32 : DP / 4;
-#define TQ_FORM(T, RC) return launch_block_scan<DELTA, KG, DP / KG, T, RC>(a, n_seqs, rec0, rec1, silu_v, rec, stream)
+#define TQ_FORM(T, RC) return launch_block_scan<DELTA, APART, KG, DP / KG, T, RC>(a, n_seqs, rec0, rec1, silu_v, rec, stream)
     const long long blocks = (long long)n_seqs * a.H * ((a.e + 128 / KG * 2 - 1) / (128 / KG * 2));
     if (blocks <= 2LL * tq_sm_count()) TQ_FORM(128, 2);
     TQ_FORM(256, 4);
@@ -529,10 +577,10 @@ static int run_block_scan(const ScanArgs& a, int n_seqs, int n_tokens, float* re
                                a, n_seqs, (int)r0, rec);
         if (st) return st;
         switch (dp) {
-            case 32: st = pick_block_scan<DELTA, 32>(a, n_seqs, (int)r0, (int)r1, silu_v, rec, stream); break;
-            case 64: st = pick_block_scan<DELTA, 64>(a, n_seqs, (int)r0, (int)r1, silu_v, rec, stream); break;
-            case 128: st = pick_block_scan<DELTA, 128>(a, n_seqs, (int)r0, (int)r1, silu_v, rec, stream); break;
-            default: st = pick_block_scan<DELTA, 256>(a, n_seqs, (int)r0, (int)r1, silu_v, rec, stream); break;
+            case 32: st = pick_block_scan<DELTA, MODE != SCAN_DELTA, 32>(a, n_seqs, (int)r0, (int)r1, silu_v, rec, stream); break;
+            case 64: st = pick_block_scan<DELTA, MODE != SCAN_DELTA, 64>(a, n_seqs, (int)r0, (int)r1, silu_v, rec, stream); break;
+            case 128: st = pick_block_scan<DELTA, MODE != SCAN_DELTA, 128>(a, n_seqs, (int)r0, (int)r1, silu_v, rec, stream); break;
+            default: st = pick_block_scan<DELTA, MODE != SCAN_DELTA, 256>(a, n_seqs, (int)r0, (int)r1, silu_v, rec, stream); break;
         }
         if (st) return st;
     }
