@@ -61,3 +61,20 @@ def test_a_cut_along_k_gives_the_same_bits_twice():
     x, w = rnd(40, 4864), rnd(896, 4864, seed=1)                          # few tiles: K is shared by a cluster
     runs = [kernels.linear(x, w) for _ in range(3)]
     assert torch.equal(runs[0], runs[1]) and torch.equal(runs[0], runs[2])
+
+
+@pytest.mark.parametrize("M,N,K,dtype", [(1, 896, 896, torch.float32), (4, 2000, 512, torch.float32), (40, 896, 4864, torch.float32),
+                                         (1, 10304, 2048, torch.bfloat16)])
+def test_a_weight_that_the_kernel_in_front_writes(M, N, K, dtype):
+    """Not a settled weight (the default): a norm kernel lets its successor start before it has written its rows."""
+    from tq_kv_b200 import kernels
+    x, g, w = rnd(M, K).to(dtype), torch.ones(K, device=DEV), torch.empty(N, K, dtype=dtype, device=DEV)
+    for i in range(5):
+        rows = rnd(N, K, seed=10 + i)
+        torch.cuda.synchronize()
+        kernels.rmsnorm(rows, g, 1e-6, w)
+        out = kernels.linear(x, w, out_dtype=torch.float32)
+        size = x.double().abs() @ w.double().abs().T
+        assert bool(((out.double() - x.double() @ w.double().T).abs() <= (K + 8) * U * size).all())
+        want = rows.double() * torch.rsqrt((rows.double() ** 2).mean(-1, keepdim=True) + 1e-6)
+        assert float((w.double() - want).abs().max()) <= 0.02 * float(want.abs().max())

@@ -1,4 +1,9 @@
 """Which decode kernel `kernels.linear` hands a bfloat16 product to (no GPU needed: the rule only looks at sizes)."""
+import ast
+import glob
+import inspect
+import os
+
 import pytest
 import torch
 
@@ -44,3 +49,18 @@ def test_which_decode_kernel_takes_a_product(rows, n, k, swiglu, after_norm, f32
     (1, 151936, 896, False, True), (1, 152064, 3584, False, True), (2, 151936, 896, False, False)])
 def test_which_products_of_one_row_run_on_the_row_kernel(rows, n, k, swiglu, want):
     assert gemm._row_takes(rows, _w(n, k), swiglu) is want
+
+
+def test_parts_say_that_their_weights_are_settled_and_nobody_else_is_taken_to():
+    """A product reads a settled weight before the kernel in front has ended: true of a model's weights, not of any w."""
+    assert inspect.signature(gemm.linear).parameters["w_settled"].default is False
+    calls = 0
+    for path in sorted(glob.glob(os.path.join(os.path.dirname(gemm.__file__), "..", "parts", "*.py"))):
+        with open(path) as f:
+            for node in ast.walk(ast.parse(f.read())):
+                if isinstance(node, ast.Call) and isinstance(node.func, ast.Attribute) and node.func.attr == "linear":
+                    calls += 1
+                    said = {k.arg: getattr(k.value, "value", None) for k in node.keywords}
+                    assert said.get("w_settled") is True, (path, node.lineno)
+                    assert isinstance(node.args[1], ast.Attribute), (path, node.lineno)        # self.w_..., a weight
+    assert calls > 30

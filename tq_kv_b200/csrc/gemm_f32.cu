@@ -32,6 +32,7 @@ struct F32TileArgs {
     const float *A, *W, *bias;
     float* C;
     int M, N, K, lda, ldw, ldc, accumulate, act, vec_out;
+    int settled;              // W was complete before the kernel in front of this one began: read it before that one ends
 };
 
 __device__ __forceinline__ void ft_copy16(float* dst, const float* src, bool ok) {
@@ -88,7 +89,8 @@ __global__ void __launch_bounds__(FT_THREADS, 2) f32_tile_kernel(const F32TileAr
         }
     };
 
-    // the weights of the first stages do not depend on the kernel before
+    // weights do not depend on the kernel before: those of the first stages are asked for at once
+    if (!a.settled) pdl_wait();
 #pragma unroll
     for (int s = 0; s < FT_STAGES - 1; ++s)
         if (s < n_steps) load_w(s);
@@ -246,15 +248,16 @@ static int f32_tile_split(long long tiles, int steps) {
 
 // gate: 0 a plain product, TQ_ACT_SILU / TQ_ACT_GELU_TANH a gated one (W has 2 N rows), TQ_ACT_SQUARE_RELU a plain one
 // with that activation.  K, lda and ldw are multiples of 4, A and W 16-byte aligned (other operands: tq_gemm_tiled).
+// settled: no kernel that may still run when this one starts writes W (it was complete before the one in front began).
 TQ_API int tq_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw,
-                       int ldc, int accumulate, int gate, cudaStream_t stream) {
+                       int ldc, int accumulate, int gate, int settled, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 4 || lda % 4 || ldw % 4 || lda < K || ldw < K || ldc < N || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) ||
         gate < 0 || gate > TQ_ACT_SQUARE_RELU)
         return (int)cudaErrorInvalidValue;
     const bool gated = gate == TQ_ACT_SILU || gate == TQ_ACT_GELU_TANH;
     F32TileArgs a{A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, gate,
-                  (ldc % 4 == 0 && ((uintptr_t)C & 15) == 0) ? 1 : 0};
+                  (ldc % 4 == 0 && ((uintptr_t)C & 15) == 0) ? 1 : 0, settled};
     // tiles of 16 or 32 rows where tiles of 64 would be mostly padding (their threads do less work per load): N = 2,048,
     // K = 5,632 at 16 rows takes 41 us in tiles of 16 and 51 in tiles of 32
     const long long pad64 = (M + 63) / 64 * 64, pad32 = (M + 31) / 32 * 32;
@@ -270,8 +273,8 @@ TQ_API int tq_gemm_f32(const float* A, const float* W, const float* bias, float*
 // ---------------------------------------------------------------------------
 // The same product for up to 8 rows (decoding in float32), bound by reading W once.  KW warps of a block make
 // NC columns (rows of W): they take 128-column pieces of K in turn, so that a block's whole share of a small W is
-// asked for at once (896 columns: one load per lane and row of W), before the kernel waits for its predecessor, whose
-// results it does not need for that; the next pieces are asked for while one is multiplied.  Every piece of A is read
+// asked for at once (896 columns: one load per lane and row of W), for a settled W before the kernel waits for its
+// predecessor, whose results it does not need for that; the next pieces are asked for while one is multiplied.  Every piece of A is read
 // once per NC columns.  The lanes' sums meet by halving (31 shuffles for 32 sums instead of 160), the warps' in
 // shared memory in the order of the warps.
 // ---------------------------------------------------------------------------
@@ -280,7 +283,7 @@ TQ_API int tq_gemm_f32(const float* A, const float* W, const float* bias, float*
 struct F32RowsArgs {
     const float *A, *W, *bias;
     float* C;
-    int M, N, K, lda, ldw, ldc, accumulate, act;
+    int M, N, K, lda, ldw, ldc, accumulate, act, settled;
 };
 
 template <int MR, int NC, int KW, bool GATED>
@@ -303,6 +306,7 @@ __global__ void __launch_bounds__(FR_WARPS * 32) f32_rows_kernel(const F32RowsAr
             w[c] = k < a.K ? *reinterpret_cast<const float4*>(wrow[c] + k) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     float4 w[NC], next[NC];
+    if (!a.settled) pdl_wait();
     if (warp < pieces) load(warp, w);
     pdl_wait();
     pdl_launch();
@@ -393,13 +397,13 @@ static int launch_f32_rows(const F32RowsArgs& a, bool gated, cudaStream_t stream
 // As tq_gemm_f32 for M <= 8 (from 9 rows on the tiles of 16 rows are faster or equal: 16 rows of N = 2,048, K = 5,632
 // take 41 us there, and took 108 in a form of this kernel).
 TQ_API int tq_gemv_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw,
-                       int ldc, int accumulate, int gate, cudaStream_t stream) {
+                       int ldc, int accumulate, int gate, int settled, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (M > 8 || K <= 0 || K % 4 || lda % 4 || ldw % 4 || (M > 1 && (lda < K || ldc < N)) || ldw < K || ((uintptr_t)A & 15) ||
         ((uintptr_t)W & 15) || gate < 0 || gate > TQ_ACT_SQUARE_RELU)
         return (int)cudaErrorInvalidValue;
     const bool gated = gate == TQ_ACT_SILU || gate == TQ_ACT_GELU_TANH;
-    const F32RowsArgs a{A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, gate};
+    const F32RowsArgs a{A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, gate, settled};
     if (M == 1) return launch_f32_rows<1>(a, gated, stream);
     if (M == 2) return launch_f32_rows<2>(a, gated, stream);
     if (M <= 4) return launch_f32_rows<4>(a, gated, stream);

@@ -5,7 +5,7 @@
 //
 // A group of KW warps makes NC = 4 neighbouring columns (rows of W; two gate and two up rows of a gated product).  A warp
 // takes pieces of 256 entries of K (16 bytes a lane and row of W) in turn, two of them in registers; the first two are
-// asked for before the kernel waits for its predecessor.  64 registers a thread keep four blocks of eight warps on an SM,
+// asked for before the kernel waits for its predecessor, if W is settled.  64 registers a thread keep four blocks of eight warps on an SM,
 // so up to 128 KB an SM are in flight.  KW is the largest of 1, 2, 4, 8 with which all warps still run at once.  The lanes'
 // sums meet by trading halves, the warps' in shared memory in warp order: no atomics, nothing to clear, and the result
 // does not depend on timing.
@@ -24,6 +24,7 @@ struct RowGemmArgs {
     const float* bias;
     void* Y;
     int N, K, ldw, accumulate, act;
+    int settled;              // W was complete before the kernel in front of this one began: read it before that one ends
 };
 
 __device__ __forceinline__ uint4 rg_load(const bf16* p) {
@@ -56,6 +57,7 @@ __global__ void __launch_bounds__(RG_WARPS * 32, 4) row_gemm_kernel(const RowGem
         for (int c = 0; c < RG_NC; ++c) w[c] = in ? rg_load(wrow[c] + piece * 256) : make_uint4(0u, 0u, 0u, 0u);
     };
     uint4 w0[RG_NC], w1[RG_NC];
+    if (!a.settled) pdl_wait();
     load(part, w0);
     load(part + KW, w1);
     pdl_wait();
@@ -135,13 +137,13 @@ static int launch_row_gemm(const RowGemmArgs& a, cudaStream_t stream) {
 // X [K] bf16, W [N, K] (or [2N, K] with a gate) bf16, Y [N] float32 or bf16.  K and ldw multiples of 8, 16-byte aligned
 // bases.  gate: 0, TQ_ACT_SILU, TQ_ACT_GELU_TANH (gated), TQ_ACT_SQUARE_RELU (plain, on its result).
 TQ_API int tq_row_gemm(const void* X, const void* W, const float* bias, void* Y, int y_dtype, int N, int K, int ldw,
-                       int accumulate, int gate, cudaStream_t stream) {
+                       int accumulate, int gate, int settled, cudaStream_t stream) {
     if (N <= 0) return 0;
     if (K <= 0 || (K & 7) || (ldw & 7) || (reinterpret_cast<uintptr_t>(X) & 15) || (reinterpret_cast<uintptr_t>(W) & 15) ||
         gate < 0 || gate > TQ_ACT_SQUARE_RELU || (y_dtype != TQ_F32 && y_dtype != TQ_BF16) ||
         (accumulate && (y_dtype != TQ_F32 || gate == TQ_ACT_SQUARE_RELU)))
         return (int)cudaErrorInvalidValue;
-    const RowGemmArgs a{(const bf16*)X, (const bf16*)W, bias, Y, N, K, ldw, accumulate, gate};
+    const RowGemmArgs a{(const bf16*)X, (const bf16*)W, bias, Y, N, K, ldw, accumulate, gate, settled};
     const bool gated = gate == TQ_ACT_SILU || gate == TQ_ACT_GELU_TANH;
     if (y_dtype == TQ_F32) return gated ? launch_row_gemm<true, float>(a, stream) : launch_row_gemm<false, float>(a, stream);
     return gated ? launch_row_gemm<true, bf16>(a, stream) : launch_row_gemm<false, bf16>(a, stream);

@@ -141,10 +141,11 @@ def skinny_gemm(x, w, out, bias=None, accumulate=False, swiglu=False, activation
     return out
 
 
-def row_gemm(x, w, out, bias=None, accumulate=False, swiglu=False, activation=elementwise.ACT_SILU):
-    """bfloat16 x [1, K] times bfloat16 w [N, K]^T on FMA units, streaming w once (csrc/row_gemm.cu); K a multiple of 8."""
+def row_gemm(x, w, out, bias=None, accumulate=False, swiglu=False, activation=elementwise.ACT_SILU, w_settled=False):
+    """bfloat16 x [1, K] times bfloat16 w [N, K]^T on FMA units, streaming w once (csrc/row_gemm.cu); K a multiple of 8.
+    `w_settled`: see `linear`."""
     check(core().tq_row_gemm(ptr(x), ptr(w), ptr(bias), ptr(out), dtype_code(out), out.shape[1], x.shape[1], w.stride(0),
-                             int(accumulate), _gate(swiglu, activation), stream()), "row_gemm")
+                             int(accumulate), _gate(swiglu, activation), int(w_settled), stream()), "row_gemm")
     return out
 
 
@@ -272,24 +273,30 @@ def _f32_ok(x, w, out) -> bool:
             and (x.shape[0] == 1 or (x.stride(0) >= K and out.stride(0) >= out.shape[1])) and w.stride(0) >= K)
 
 
-def gemm_f32(x, w, out, bias=None, accumulate=False, swiglu=False, activation=elementwise.ACT_SILU):
+def gemm_f32(x, w, out, bias=None, accumulate=False, swiglu=False, activation=elementwise.ACT_SILU, w_settled=False):
     """float32 x [M, K] times w [N, K]^T on FMA units (csrc/gemm_f32.cu): up to 8 rows by the kernel that streams w
-    once, more by tiles."""
+    once, more by tiles.  `w_settled`: see `linear`."""
     M, K = x.shape
     fn = core().tq_gemv_f32 if M <= F32_ROW_KERNEL_MAX_ROWS else core().tq_gemm_f32
     check(fn(ptr(x), ptr(w), ptr(bias), ptr(out), M, out.shape[1], K, x.stride(0), w.stride(0), out.stride(0),
-             int(accumulate), _gate(swiglu, activation), stream()), "gemm_f32")
+             int(accumulate), _gate(swiglu, activation), int(w_settled), stream()), "gemm_f32")
     return out
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = None,
            out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
-           accumulate: bool = False, swiglu: bool = False, activation: int = elementwise.ACT_SILU) -> torch.Tensor:
+           accumulate: bool = False, swiglu: bool = False, activation: int = elementwise.ACT_SILU,
+           w_settled: bool = False) -> torch.Tensor:
     """y = x · w^T (+ bias); with `swiglu`, w holds gate rows then up rows and
     y = act(x · gate^T) * (x · up^T), act being silu unless `activation` names another; without it and with
     `activation` ACT_SQUARE_RELU, y = max(x · w^T + bias, 0)^2 (not with `accumulate`); with `accumulate`, `out` (float32) gets
     y added to it.  x [M, K], w [N, K] (or [2N, K]); float32 accumulation
-    throughout."""
+    throughout.
+
+    `w_settled`: w was complete before the kernel in front of this product began, as a model's weights are.  The
+    product may then start to read it while that kernel still runs; without it float32 products and the row kernel
+    wait first.  The bfloat16 decode kernels (up to 64 rows) always read ahead: a bfloat16 w that a kernel of this
+    package makes has to have another kernel behind it before its product."""
     pending = x if isinstance(x, PendingNorm) else None
     relu2 = activation == elementwise.ACT_SQUARE_RELU
     if relu2 and (swiglu or accumulate):
@@ -322,7 +329,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = N
     if (_row_takes(M, w, bool(swiglu)) and USE_TCGEN05 and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K % 8 == 0
             and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and out.dtype in (torch.float32, torch.bfloat16) and (not accumulate or out.dtype == torch.float32)):
-        return row_gemm(x, w, out, bias, accumulate, swiglu, activation)
+        return row_gemm(x, w, out, bias, accumulate, swiglu, activation, w_settled)
     # decoding: the TMA-fed tcgen05 kernel or the mma.sync kernel (_tc_takes says which, where both can)
     if (USE_TCGEN05 and M <= SKINNY_MAX_ROWS and _tc_ok(x, w, out, swiglu)
             and (not accumulate or out.dtype == torch.float32) and not (relu2 and out.dtype != torch.bfloat16)
@@ -332,7 +339,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = N
     if _skinny_ok(x, w):
         return skinny_gemm(x, w, out, bias, accumulate, swiglu, activation)
     if _f32_ok(x, w, out):
-        return gemm_f32(x, w, out, bias, accumulate, swiglu, activation)
+        return gemm_f32(x, w, out, bias, accumulate, swiglu, activation, w_settled)
     if M <= ROW_KERNEL_MAX_ROWS:
         return gemv_rows(x, w, out, bias, accumulate, swiglu, activation)
 

@@ -121,9 +121,9 @@ class GQAttention(Mixer):
             if dirty[0]:                                   # a step failed between the product and the rotary kernel
                 buf.zero_()
             dirty[0] = True
-            qkv = kernels.linear(x, self.w_qkv, out=buf[:T], accumulate=True)
+            qkv = kernels.linear(x, self.w_qkv, out=buf[:T], accumulate=True, w_settled=True)
         else:
-            qkv = kernels.linear(x, self.w_qkv, out_dtype=torch.float32)
+            qkv = kernels.linear(x, self.w_qkv, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
         q = torch.empty((T, self.q_width), dtype=act, device=dev)
         k = torch.empty((T, self.kv_width), dtype=act, device=dev) if packed else None
@@ -151,5 +151,5 @@ class GQAttention(Mixer):
                               table_width=kv.table_width, ring_pages=kv.ring_pages, page_tokens=kv.page_tokens,
                               n_splits=n_splits, scratch=scratch, **common)
         kernels.mark("attention")
-        kernels.linear(out, self.w_o, bias=self.b_o, out=residual, accumulate=True)
+        kernels.linear(out, self.w_o, bias=self.b_o, out=residual, accumulate=True, w_settled=True)
         kernels.mark("o")

@@ -102,7 +102,7 @@ class ChannelDeltaMixer(Mixer):
     def forward(self, x, ctx: StepContext, residual):
         b, dev = ctx.batch, residual.device
         qk, vw, C, H = self.qk, self.vw, self.conv_channels, self.heads
-        proj = kernels.linear(x, self.w_in, bias=self.bias, out_dtype=torch.float32)
+        proj = kernels.linear(x, self.w_in, bias=self.bias, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
         if self.rider is not None:
             ctx.rider_out = proj[:, self.off_rider:self.off_a]
@@ -131,5 +131,5 @@ class ChannelDeltaMixer(Mixer):
         y = torch.empty((T, vw), dtype=ctx.runtime.act_dtype, device=dev)
         kernels.group_rmsnorm(o, self.norm_w, self.eps, y, groups=H, gate=gate)
         kernels.mark("head_norm")
-        kernels.linear(y, self.w_o, out=residual, accumulate=not ctx.store_result)
+        kernels.linear(y, self.w_o, out=residual, accumulate=not ctx.store_result, w_settled=True)
         kernels.mark("o")

@@ -63,7 +63,7 @@ class DecayedStateMixer(Mixer):
     def forward(self, x, ctx: StepContext, residual):
         b, dev = ctx.batch, residual.device
         act = ctx.runtime.act_dtype
-        proj = kernels.linear(x, self.w_in, out_dtype=torch.float32)
+        proj = kernels.linear(x, self.w_in, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
         T = proj.shape[0]
         o = torch.empty((T, self.vw), dtype=torch.float32, device=dev)
@@ -74,5 +74,5 @@ class DecayedStateMixer(Mixer):
         y = torch.empty((T, self.vw), dtype=act, device=dev)
         kernels.group_rmsnorm(o, self.norm_w, self.eps, y, groups=1, gate=proj[:, 2 * self.qk + self.vw:])
         kernels.mark("norms")
-        kernels.linear(y, self.w_o, out=residual, accumulate=True)
+        kernels.linear(y, self.w_o, out=residual, accumulate=True, w_settled=True)
         kernels.mark("o")

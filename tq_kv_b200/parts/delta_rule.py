@@ -89,12 +89,12 @@ class DeltaRuleMixer(Mixer):
     def forward(self, x, ctx: StepContext, residual):
         b, n, dev = ctx.batch, self.inner, residual.device
         act = ctx.runtime.act_dtype
-        proj = kernels.linear(x, self.w_in, bias=self.b_in, out_dtype=torch.float32)
+        proj = kernels.linear(x, self.w_in, bias=self.b_in, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
         T = proj.shape[0]
         low = torch.empty((T, self.rank), dtype=torch.float32 if self.decay_in_float32 else act, device=dev)
         kernels.tanh_rows(proj[:, 5 * n:], low)
-        decay_logit = kernels.linear(low, self.w_decay, bias=self.b_decay, out_dtype=torch.float32)
+        decay_logit = kernels.linear(low, self.w_decay, bias=self.b_decay, out_dtype=torch.float32, w_settled=True)
         kernels.mark("decay")
         o = torch.empty((T, n), dtype=torch.float32, device=dev)
         kernels.linear_scan(proj, ctx.state, b.cu_seqlens, b.slots, o, n_seqs=b.n_seqs, heads=self.heads,
@@ -104,5 +104,5 @@ class DeltaRuleMixer(Mixer):
         y = torch.empty((T, n), dtype=act, device=dev)
         kernels.group_rmsnorm(o, self.norm_w, self.eps, y, groups=self.heads, gate=proj[:, 3 * n:4 * n])
         kernels.mark("norms")
-        kernels.linear(y, self.w_o, out=residual, accumulate=True)
+        kernels.linear(y, self.w_o, out=residual, accumulate=True, w_settled=True)
         kernels.mark("o")

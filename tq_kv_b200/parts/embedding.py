@@ -83,7 +83,7 @@ class LMHead(Part):
 
     def forward(self, normed_rows: torch.Tensor) -> torch.Tensor:
         """float32 logits [rows, vocab] of already normed rows."""
-        logits = kernels.linear(normed_rows, self.weight, out_dtype=torch.float32)
+        logits = kernels.linear(normed_rows, self.weight, out_dtype=torch.float32, w_settled=True)
         if self.logit_scale != 1.0:
             kernels.scale_inplace(logits, self.logit_scale)
         if self.logit_softcap is not None:

@@ -46,9 +46,9 @@ class SwiGLU(FeedForward):
 
     def forward(self, x, ctx: StepContext, residual):
         act = kernels.linear(x, self.w_gate_up, swiglu=True, activation=self.activation,
-                             out_dtype=ctx.runtime.act_dtype)
+                             out_dtype=ctx.runtime.act_dtype, w_settled=True)
         kernels.mark("gate_up")
-        kernels.linear(act, self.w_down, out=residual, accumulate=not ctx.store_result)
+        kernels.linear(act, self.w_down, out=residual, accumulate=not ctx.store_result, w_settled=True)
         kernels.mark("down")
 
 
@@ -78,7 +78,7 @@ class PlainFeedForward(FeedForward):
         self.w_down = tensors[self._n("down")].contiguous()
 
     def forward(self, x, ctx: StepContext, residual):
-        act = kernels.linear(x, self.w_up, activation=self.activation, out_dtype=ctx.runtime.act_dtype)
+        act = kernels.linear(x, self.w_up, activation=self.activation, out_dtype=ctx.runtime.act_dtype, w_settled=True)
         kernels.mark("up")
-        kernels.linear(act, self.w_down, out=residual, accumulate=not ctx.store_result)
+        kernels.linear(act, self.w_down, out=residual, accumulate=not ctx.store_result, w_settled=True)
         kernels.mark("down")

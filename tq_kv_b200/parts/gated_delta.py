@@ -81,7 +81,7 @@ class GatedDeltaMixer(Mixer):
         b, dev = ctx.batch, residual.device
         act = ctx.runtime.act_dtype
         qk, vw, C, H = self.qk, self.vw, self.conv_channels, self.heads
-        proj = kernels.linear(x, self.w_in, out_dtype=torch.float32)
+        proj = kernels.linear(x, self.w_in, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
         T = proj.shape[0]
         single = b.single_tokens
@@ -102,5 +102,5 @@ class GatedDeltaMixer(Mixer):
         y = torch.empty((T, vw), dtype=act, device=dev)
         kernels.group_rmsnorm(o, self.norm_w, self.eps, y, groups=H, gate=proj[:, C + 2 * H:], gate_mode=kernels.GATE_SILU)
         kernels.mark("norms")
-        kernels.linear(y, self.w_o, out=residual, accumulate=True)
+        kernels.linear(y, self.w_o, out=residual, accumulate=True, w_settled=True)
         kernels.mark("o")

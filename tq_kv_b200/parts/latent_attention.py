@@ -167,7 +167,7 @@ class LatentAttention(Mixer):
         b, kv, dev = ctx.batch, ctx.kv, residual.device
         act = ctx.runtime.act_dtype
         H, row = self.heads, self.row
-        proj = kernels.linear(x, self.w_in, out_dtype=torch.float32)
+        proj = kernels.linear(x, self.w_in, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
         T = proj.shape[0]
         owns = kv is not None and kv.writes and not self.shared_kv
@@ -192,7 +192,7 @@ class LatentAttention(Mixer):
                                 ring_pages=kv.ring_pages if owns else 0, out_dtype=act, **rot)
             kernels.mark("rotary")
         if self.q_rank:
-            q = kernels.linear(cq, self.w_uq, out_dtype=act if packed and self.plain_heads else torch.float32)
+            q = kernels.linear(cq, self.w_uq, out_dtype=act if packed and self.plain_heads else torch.float32, w_settled=True)
             kernels.mark("qkv")
         else:
             q = proj[:, :self.q_cols]
@@ -208,11 +208,11 @@ class LatentAttention(Mixer):
             if self.plain_heads:
                 # nothing to turn and nothing to fill up: the products leave the heads as the attention takes them
                 qh = q
-                kh = kernels.linear(lat, self.w_uk, out_dtype=act)
-                vh = kernels.linear(lat, self.w_uv, out_dtype=act)
+                kh = kernels.linear(lat, self.w_uk, out_dtype=act, w_settled=True)
+                vh = kernels.linear(lat, self.w_uv, out_dtype=act, w_settled=True)
                 kernels.mark("qkv")
             else:
-                kfv = kernels.linear(lat, self.w_ukv, out_dtype=torch.float32)
+                kfv = kernels.linear(lat, self.w_ukv, out_dtype=torch.float32, w_settled=True)
                 kernels.mark("qkv")
                 qh, kh, vh = (torch.empty((T, H * hw), dtype=act, device=dev) for _ in range(3))
                 kernels.latent_heads(q, kfv, rows, qh, kh, vh, heads=H, dim=self.dim, rot_dim=self.rot_dim,
@@ -228,7 +228,7 @@ class LatentAttention(Mixer):
                 kernels.latent_expand(oh, None, y, heads=H, kv_rank=hw, row_width=hw, value_dim=self.value_dim, gate=gate,
                                       head_gate=self.head_gate)
                 kernels.mark("rotary")
-            kernels.linear(y, self.w_o, out=residual, accumulate=not ctx.store_result)
+            kernels.linear(y, self.w_o, out=residual, accumulate=not ctx.store_result, w_settled=True)
             kernels.mark("o")
             return
         qa = torch.empty((T, H * row), dtype=act, device=dev)
@@ -248,7 +248,7 @@ class LatentAttention(Mixer):
         kernels.latent_expand(lat, self.w_uv, y, heads=H, kv_rank=self.kv_rank, row_width=row,
                               value_dim=self.value_dim, gate=gate, head_gate=self.head_gate)
         kernels.mark("rotary")
-        kernels.linear(y, self.w_o, out=residual, accumulate=not ctx.store_result)
+        kernels.linear(y, self.w_o, out=residual, accumulate=not ctx.store_result, w_settled=True)
         kernels.mark("o")
 
     def _attend(self, q, out, width, gate=None, **kw):

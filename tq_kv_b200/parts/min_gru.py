@@ -55,7 +55,7 @@ class MinGRUMixer(Mixer):
         return self.w_in, self.bias
 
     def forward(self, x, ctx: StepContext, residual):
-        proj = kernels.linear(x, self.w_in, bias=self.bias, out_dtype=torch.float32)
+        proj = kernels.linear(x, self.w_in, bias=self.bias, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
         self.run(proj, ctx, residual, accumulate=not ctx.store_result)
 
@@ -66,5 +66,5 @@ class MinGRUMixer(Mixer):
         kernels.gru_scan(proj[:, :n], proj[:, s:s + n], proj[:, 2 * s:2 * s + n], ctx.state, b.cu_seqlens, b.slots, y,
                          n_seqs=b.n_seqs, scale=self.result_scale, single_tokens=b.single_tokens)
         kernels.mark("gru")
-        kernels.linear(y, self.w_o, out=residual, accumulate=accumulate)
+        kernels.linear(y, self.w_o, out=residual, accumulate=accumulate, w_settled=True)
         kernels.mark("o")

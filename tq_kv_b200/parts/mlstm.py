@@ -82,7 +82,7 @@ class MatrixMemoryMixer(Mixer):
     def forward(self, x, ctx: StepContext, residual):
         b, dev = ctx.batch, residual.device
         H, d, e, ea = self.heads, self.key_dim, self.value_dim, self.value_cols
-        proj = kernels.linear(x, self.w_in, bias=self.bias, out_dtype=torch.float32)
+        proj = kernels.linear(x, self.w_in, bias=self.bias, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
         T = proj.shape[0]
         scal = kernels.mlstm_gates(proj[:, self.off_i:self.off_i + H], proj[:, self.off_f:self.off_f + H], self.gate_cap,
@@ -97,5 +97,5 @@ class MatrixMemoryMixer(Mixer):
         kernels.mlstm_read(o, scal, proj[:, self.off_g:self.off_i], self.norm_w, y, heads=H, value_dim=e,
                            q_scale=d ** -0.5, floor=self.read_floor, eps=self.eps)
         kernels.mark("norms")
-        kernels.linear(y, self.w_o, out=residual, accumulate=not ctx.store_result)
+        kernels.linear(y, self.w_o, out=residual, accumulate=not ctx.store_result, w_settled=True)
         kernels.mark("o")

@@ -133,7 +133,7 @@ class SublayerResult(Part):
     def gate_logits(self, x) -> Optional[torch.Tensor]:
         if self.w_gate is None:
             return None
-        return kernels.linear(x, self.w_gate, bias=self.gate_bias, out_dtype=torch.float32)
+        return kernels.linear(x, self.w_gate, bias=self.gate_bias, out_dtype=torch.float32, w_settled=True)
 
 
 class StreamsBlock:

@@ -157,18 +157,18 @@ class TableExperts(FeedForward):
         if self.routing == "table":
             choice = kernels.table_choice(ctx.batch.tokens, self.table, self.n_experts)
         elif self.routing == "group_router":
-            proj = kernels.linear(x, self.w_router, bias=self.router_bias, out_dtype=torch.float32)
+            proj = kernels.linear(x, self.w_router, bias=self.router_bias, out_dtype=torch.float32, w_settled=True)
             kernels.mark("router")
             if self.rider is not None:
                 ctx.rider_out = proj[:, :self.router_col]
             choice, weights = kernels.group_router_choice(proj[:, self.router_col:self.router_col + self.n_experts],
                                                           self.top, self.correction, self.groups, self.keep_groups)
         elif self.routing == "softmax_router":
-            proj = kernels.linear(x, self.w_router, bias=self.router_bias, out_dtype=torch.float32)
+            proj = kernels.linear(x, self.w_router, bias=self.router_bias, out_dtype=torch.float32, w_settled=True)
             kernels.mark("router")
             choice, weights = kernels.router_choice(proj[:, :self.n_experts], self.top, softmax=True)
         else:
-            logits = kernels.linear(x, self.w_router, out_dtype=torch.float32)
+            logits = kernels.linear(x, self.w_router, out_dtype=torch.float32, w_settled=True)
             choice, weights = kernels.router_choice(logits, self.top, self.router_scale, self.weight_sum_floor)
         T = x.shape[0]
         shared = {}
@@ -188,10 +188,10 @@ class TableExperts(FeedForward):
     def _shared_result(self, x, ctx, residual=None):
         """The shared expert's result, added into `residual` or (none given) in float32 rows of its own."""
         act = kernels.linear(x, self.w_shared_gate_up, swiglu=self.gated, out_dtype=ctx.runtime.act_dtype,
-                             activation=kernels.ACT_SILU if self.gated else kernels.ACT_SQUARE_RELU)
+                             activation=kernels.ACT_SILU if self.gated else kernels.ACT_SQUARE_RELU, w_settled=True)
         if residual is None:
-            out = kernels.linear(act, self.w_shared_down, out_dtype=torch.float32)
+            out = kernels.linear(act, self.w_shared_down, out_dtype=torch.float32, w_settled=True)
         else:
-            out = kernels.linear(act, self.w_shared_down, out=residual, accumulate=True)
+            out = kernels.linear(act, self.w_shared_down, out=residual, accumulate=True, w_settled=True)
         kernels.mark("shared_expert")
         return out

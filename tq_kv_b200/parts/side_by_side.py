@@ -99,7 +99,7 @@ class SideBySideMixer(Mixer):
         if isinstance(x, kernels.PendingNorm):
             x = x.materialize()
         if self.one_product:
-            proj = kernels.linear(x, self.w_in, bias=self.bias, out_dtype=torch.float32)
+            proj = kernels.linear(x, self.w_in, bias=self.bias, out_dtype=torch.float32, w_settled=True)
             kernels.mark("qkv")
             for i, b in enumerate(self.branches):
                 lo, hi = self.columns[i]

@@ -145,7 +145,7 @@ class SigmoidAttention(Mixer):
     def forward(self, x, ctx: StepContext, residual):
         b, kv, dev = ctx.batch, ctx.kv, residual.device
         act = ctx.runtime.act_dtype
-        proj = kernels.linear(x, self.w_in, bias=self.b_in, out_dtype=torch.float32)
+        proj = kernels.linear(x, self.w_in, bias=self.b_in, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
         T = proj.shape[0]
         owns = kv is not None and kv.writes
@@ -178,5 +178,5 @@ class SigmoidAttention(Mixer):
                                       table_width=kv.table_width, page_tokens=kv.page_tokens, n_splits=n_splits,
                                       scratch=scratch, **common)
         kernels.mark("attention")
-        kernels.linear(out, self.w_o, out=residual, accumulate=True)
+        kernels.linear(out, self.w_o, out=residual, accumulate=True, w_settled=True)
         kernels.mark("o")

@@ -287,7 +287,7 @@ class SoftmaxAttention(Mixer):
         return self.w_in, None
 
     def forward(self, x, ctx: StepContext, residual):
-        proj = kernels.linear(x, self.w_in, out_dtype=torch.float32)
+        proj = kernels.linear(x, self.w_in, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
         self.run(proj, ctx, residual, accumulate=not ctx.store_result)
 
@@ -357,5 +357,5 @@ class SoftmaxAttention(Mixer):
             kernels.mark("difference")
         elif self.head_gate:
             kernels.sigmoid_gate(out, gate)
-        kernels.linear(out, self.w_o, out=residual, accumulate=accumulate)
+        kernels.linear(out, self.w_o, out=residual, accumulate=accumulate, w_settled=True)
         kernels.mark("o")

@@ -77,7 +77,7 @@ class StateSpaceMixer(Mixer):
         b, dev = ctx.batch, residual.device
         act = ctx.runtime.act_dtype
         inner, bc, C, H = self.inner, self.bc, self.conv_channels, self.heads
-        proj = kernels.linear(x, self.w_in, out_dtype=torch.float32)
+        proj = kernels.linear(x, self.w_in, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
         T = proj.shape[0]
         single = b.single_tokens
@@ -98,5 +98,5 @@ class StateSpaceMixer(Mixer):
         kernels.group_rmsnorm(o, self.norm_w, self.eps, y, groups=self.norm_groups, gate=proj[:, :inner],
                               gate_mode=kernels.GATE_SILU_FIRST)
         kernels.mark("norms")
-        kernels.linear(y, self.w_o, out=residual, accumulate=True)
+        kernels.linear(y, self.w_o, out=residual, accumulate=True, w_settled=True)
         kernels.mark("o")
