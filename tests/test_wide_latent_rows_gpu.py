@@ -96,3 +96,42 @@ def test_a_weight_keeps_its_24_bits():
     w = (16.0 * r[:, 0]).softmax(0)
     want = w @ r
     assert float((out[0].double() - want).abs()[1]) <= 2.0 ** -8 * float(want[1].abs())
+
+
+def common_args(hd, heads, q_pages, poss, seqs, cu, st, width, table):
+    return dict(n_heads=heads, n_kv_heads=1, head_dim=hd, tok_pos=poss, tok_seq=seqs, cu_seqlens=cu, start_pos=st, window=None,
+                k_pages=q_pages, v_pages=q_pages, block_table=table, table_width=width)
+
+
+@pytest.mark.parametrize("hd", [192, 256])
+def test_rows_that_the_kernel_in_front_writes(hd):
+    """All cached rows, not the newest alone, come from a kernel that lets its successor start before it has written them."""
+    from tq_kv_b200 import kernels
+    q, pages, table, width, poss, seqs, cu, st = case(hd, 16, [3000] * 8, [1] * 8, seed=hd)
+    scratch = torch.empty(kernels.split_scratch_floats(8, 16, hd, 6) + 1, device=DEV)
+    g, flat = torch.ones(hd, device=DEV), pages.view(-1, hd)
+    for i in range(5):
+        rows = torch.randn(flat.shape, generator=torch.Generator().manual_seed(i)).to(DEV)
+        out = torch.empty_like(q)
+        torch.cuda.synchronize()
+        kernels.rmsnorm(rows, g, 1e-6, flat)
+        kernels.attention(q, out, n_splits=6, scratch=scratch, **common_args(hd, 16, pages, poss, seqs, cu, st, width, table))
+        want = exact(q, pages, table, poss, seqs, 16, hd, hd ** -0.5, None, None)
+        assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5).all())
+
+
+@pytest.mark.parametrize("hd", [192, 256])
+def test_a_query_off_the_16_byte_boundary(hd):
+    """The general kernel takes it, as it did before these rows had a kernel of their own."""
+    from tq_kv_b200 import kernels
+    q, pages, table, width, poss, seqs, cu, st = case(hd, 5, [0, 70, 300], [1, 1, 1], seed=1)
+    shifted = torch.empty(q.numel() + 1, dtype=q.dtype, device=DEV)[1:].view(q.shape).copy_(q)
+    assert shifted.data_ptr() % 16 and shifted.is_contiguous()
+    got, aligned = torch.empty_like(q), torch.empty_like(q)
+    kw = common_args(hd, 5, pages, poss, seqs, cu, st, width, table)
+    kernels.attention(shifted, got, **kw)
+    kernels.attention(q, aligned, use_flash=False, **kw)
+    assert torch.equal(got, aligned)
+    ext = {k: v for k, v in kw.items() if k != "head_dim"}
+    kernels.attention_ext(shifted, got, key_dim=hd, value_dim=hd, scale=hd ** -0.5, **ext)
+    assert torch.equal(got, aligned)

@@ -107,6 +107,7 @@ flash_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gid = lane >> 2, tid4 = lane & 3;
     const int n_rep = nh / nkv;
+    if constexpr (WIDE) pdl_wait();      // nothing is read ahead: these rows' kernel before was ordered by the stream
     const int pos = tok_pos[t];
     const int b = tok_seq[t];
     int lo_all = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
@@ -434,13 +435,13 @@ static int launch_flash_decode(const bf16* q, const bf16* kp, const bf16* vp, co
 }
 
 // Returns cudaErrorNotSupported (801) for shapes outside this kernel's reach
-// (head_dim not in {32, 64, 96, 128}, or in {192, 256} with values that are the keys; q heads per key/value head that do not
+// (head_dim not in {32, 64, 96, 128}, or in {192, 256} with values that are the keys and a q on a 16-byte boundary; q heads per key/value head that do not
 // cut into equal groups of at most 16, pages of another size); the caller then uses the general kernel.
 //
 // `early_start`: launch the kernel so that it may begin while its predecessor in the stream still runs
 // (programmatic dependent launch).  Its blocks then read the positions, the block table and every key older than
-// the token's own before the predecessor has ended; that is right only if the predecessor writes nothing but q
-// and each token's newest key, as the kernels of a decode step do.  With 0 the kernel starts after everything
+// the token's own before the predecessor has ended (rows of up to 128 entries do; wider ones wait first); that is right only
+// if the predecessor writes nothing but q and each token's newest key, as the kernels of a decode step do.  With 0 the kernel starts after everything
 // before it in the stream has completed, whatever that was.
 static int flash_decode_launch(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                                int table_width, int ring_pages, int page_tokens, const int* tok_pos,
@@ -457,6 +458,7 @@ static int flash_decode_launch(const void* q, const void* k_pages, const void* v
     if (nkv > 65535 || n_splits > 65535) return (int)cudaErrorNotSupported;
     if (n_splits < 1 || (n_splits > 1 && (!part_acc || !part_ml))) return (int)cudaErrorInvalidValue;
     const bool same = k_pages == v_pages;               // the values are the keys: one tile per stage
+    const bool wide_ok = same && (reinterpret_cast<uintptr_t>(q) & 15) == 0;      // (wide rows: q goes in 16-byte pieces)
 #define TQ_FD_ARGS (const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, block_table, table_width, ring_pages,      \
                    tok_pos, tok_seq, window, scale, (bf16*)out, part_acc, part_ml, n_tokens, nh, nkv, n_splits,            \
                    early_start ? TQ_PDL_FLASH_DECODE : 0, stream, nullptr, 0, nullptr, 0, kv_div
@@ -468,8 +470,8 @@ static int flash_decode_launch(const void* q, const void* k_pages, const void* v
         TQ_FD(64);
         TQ_FD(96);
         TQ_FD(128);
-        case 192: return same ? launch_flash_decode<192, FD_SOFTMAX, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
-        case 256: return same ? launch_flash_decode<256, FD_SOFTMAX, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
+        case 192: return wide_ok ? launch_flash_decode<192, FD_SOFTMAX, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
+        case 256: return wide_ok ? launch_flash_decode<256, FD_SOFTMAX, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
         default: return (int)cudaErrorNotSupported;
     }
 #undef TQ_FD_ARGS
@@ -534,6 +536,7 @@ TQ_API int tq_flash_decode_ext(const void* q, const void* k_pages, const void* v
     if (chunk < 0 || (chunk > 0 && window > 0)) return (int)cudaErrorInvalidValue;
     const FdOptions opt{scale, softcap, slopes, window > 0 ? keep_first : 0, sinks, chunk};
     const bool same = k_pages == v_pages;
+    const bool wide_ok = same && (reinterpret_cast<uintptr_t>(q) & 15) == 0;      // (wide rows: q goes in 16-byte pieces)
 #define TQ_FD_ARGS (const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, block_table, table_width, ring_pages,      \
                    tok_pos, tok_seq, window, scale, (bf16*)out, part_acc, part_ml, n_tokens, nh, nkv, n_splits,            \
                    TQ_PDL_FLASH_DECODE, stream, nullptr, 0, nullptr, 0, kv_div, opt
@@ -545,8 +548,8 @@ TQ_API int tq_flash_decode_ext(const void* q, const void* k_pages, const void* v
         TQ_FD(64);
         TQ_FD(96);
         TQ_FD(128);
-        case 192: return same ? launch_flash_decode<192, FD_SOFTMAX_EXT, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
-        case 256: return same ? launch_flash_decode<256, FD_SOFTMAX_EXT, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
+        case 192: return wide_ok ? launch_flash_decode<192, FD_SOFTMAX_EXT, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
+        case 256: return wide_ok ? launch_flash_decode<256, FD_SOFTMAX_EXT, 0>(TQ_FD_ARGS) : (int)cudaErrorNotSupported;
         default: return (int)cudaErrorNotSupported;
     }
 #undef TQ_FD_ARGS
