@@ -135,3 +135,35 @@ def test_a_query_off_the_16_byte_boundary(hd):
     ext = {k: v for k, v in kw.items() if k != "head_dim"}
     kernels.attention_ext(shifted, got, key_dim=hd, value_dim=hd, scale=hd ** -0.5, **ext)
     assert torch.equal(got, aligned)
+
+
+@pytest.mark.parametrize("hd", [192, 256])
+@pytest.mark.parametrize("n_splits", [1, 4])
+@pytest.mark.parametrize("softcap", [None, 50.0])
+def test_parts_that_leave_unmerged_come_from_the_general_kernel(hd, n_splits, softcap):
+    """They are float32 results, and its sums are the more exact ones."""
+    from tq_kv_b200 import kernels
+    H = 16
+    q, pages, table, width, poss, seqs, cu, st = case(hd, H, [3000, 500, 64, 40], [1] * 4, seed=hd)
+    got = [kernels.attention_ext(q, None, n_heads=H, n_kv_heads=1, key_dim=hd, value_dim=hd, tok_pos=poss, tok_seq=seqs,
+                                 cu_seqlens=cu, start_pos=st, scale=hd ** -0.5, softcap=softcap, k_pages=pages, v_pages=pages,
+                                 block_table=table, table_width=width, n_splits=n_splits, unmerged=True, use_fast=fast)
+           for fast in (True, False)]
+    assert got[0][2] == got[1][2] == n_splits and torch.equal(got[0][1], got[1][1])
+    full = got[0][1].reshape(4, H, n_splits, 2)[..., 1] > 0                # (a split without keys holds nothing)
+    assert torch.equal(got[0][0].reshape(4, H, n_splits, hd)[full], got[1][0].reshape(4, H, n_splits, hd)[full])
+
+
+@pytest.mark.parametrize("hd", [192, 256])
+def test_a_cap_on_the_scores(hd):
+    from tq_kv_b200 import kernels
+    H, starts = 16, [700, 64]
+    q, pages, table, width, poss, seqs, cu, st = case(hd, H, starts, [1] * 2, seed=hd, sharp=3.0)
+    out = torch.empty_like(q)
+    kernels.attention_ext(q, out, n_heads=H, n_kv_heads=1, key_dim=hd, value_dim=hd, tok_pos=poss, tok_seq=seqs, cu_seqlens=cu,
+                          start_pos=st, scale=hd ** -0.5, softcap=20.0, k_pages=pages, v_pages=pages, block_table=table,
+                          table_width=width)
+    for t, p in enumerate(starts):
+        rows = pages[table[t].long()].reshape(-1, hd)[:p + 1].double()
+        want = ((20.0 * torch.tanh(q[t].double().reshape(H, hd) @ rows.T * hd ** -0.5 / 20.0)).softmax(-1) @ rows).reshape(-1)
+        assert bool(((out[t].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5).all())

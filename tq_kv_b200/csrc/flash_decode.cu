@@ -536,7 +536,10 @@ TQ_API int tq_flash_decode_ext(const void* q, const void* k_pages, const void* v
     if (chunk < 0 || (chunk > 0 && window > 0)) return (int)cudaErrorInvalidValue;
     const FdOptions opt{scale, softcap, slopes, window > 0 ? keep_first : 0, sinks, chunk};
     const bool same = k_pages == v_pages;
-    const bool wide_ok = same && (reinterpret_cast<uintptr_t>(q) & 15) == 0;      // (wide rows: q goes in 16-byte pieces)
+    // Wide rows: q goes in 16-byte pieces; and the float32 parts that a caller takes as they are come from the general kernel,
+    // whose sums are closer to 64 bits (3,000 keys in one piece: 1.9e-7 of the norm, here 3.9e-7 and with a cap of 50
+    // 2.0e-6; a bfloat16 result keeps 2e-3)
+    const bool wide_ok = same && (reinterpret_cast<uintptr_t>(q) & 15) == 0 && out;
 #define TQ_FD_ARGS (const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, block_table, table_width, ring_pages,      \
                    tok_pos, tok_seq, window, scale, (bf16*)out, part_acc, part_ml, n_tokens, nh, nkv, n_splits,            \
                    TQ_PDL_FLASH_DECODE, stream, nullptr, 0, nullptr, 0, kv_div, opt
