@@ -257,8 +257,13 @@ attention_merge_kernel(const float* __restrict__ part_acc, const float* __restri
             a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
         }
         TC* o = out + ((size_t)blockIdx.x * nh + blockIdx.y) * hd + piece * 4;
-        store2_f32<TC>(o, a.x / l, a.y / l);
-        store2_f32<TC>(o + 2, a.z / l, a.w / l);
+        if ((reinterpret_cast<uintptr_t>(out) & (2 * sizeof(TC) - 1)) == 0) {
+            store2_f32<TC>(o, a.x / l, a.y / l);
+            store2_f32<TC>(o + 2, a.z / l, a.w / l);
+        } else {                                        // a result that starts between two pairs
+            o[0] = from_f32<TC>(a.x / l); o[1] = from_f32<TC>(a.y / l);
+            o[2] = from_f32<TC>(a.z / l); o[3] = from_f32<TC>(a.w / l);
+        }
     }
 }
 
