@@ -78,3 +78,18 @@ def test_a_weight_that_the_kernel_in_front_writes(M, N, K, dtype):
         assert bool(((out.double() - x.double() @ w.double().T).abs() <= (K + 8) * U * size).all())
         want = rows.double() * torch.rsqrt((rows.double() ** 2).mean(-1, keepdim=True) + 1e-6)
         assert float((w.double() - want).abs().max()) <= 0.02 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_more_columns_than_a_grid_has_tiles_for(swiglu):
+    """The general kernels take them, as they did before."""
+    from tq_kv_b200 import kernels
+    N = 64 * 65535 + 1
+    x, w = rnd(20, 4), rnd(1000, 4, seed=1).repeat(N // 500 + 1, 1)[:2 * N if swiglu else N]
+    out = kernels.linear(x, w, swiglu=swiglu)
+    z = x.double() @ w[:1000].double().T                                   # (the weight's rows repeat every 1,000)
+    at = torch.tensor([0, 1, 999, 64 * 65535 - 1, N - 1], device=DEV)
+    want = z[:, at % 1000]
+    if swiglu:
+        want = torch.nn.functional.silu(want) * z[:, (at + N) % 1000]
+    assert float((out[:, at].double() - want).abs().max()) <= 64 * U * float(want.abs().max())

@@ -64,3 +64,9 @@ def test_parts_say_that_their_weights_are_settled_and_nobody_else_is_taken_to():
                     assert said.get("w_settled") is True, (path, node.lineno)
                     assert isinstance(node.args[1], ast.Attribute), (path, node.lineno)        # self.w_..., a weight
     assert calls > 30
+
+
+@pytest.mark.parametrize("rows, n, want", [(8, 5_000_000, True), (9, 64 * 65535, True), (9, 64 * 65535 + 1, False), (300, 5_000_000, False)])
+def test_float32_products_with_more_columns_than_a_grid_has_tiles_for(rows, n, want):
+    x, w, out = (torch.empty(s, device="meta") for s in ((rows, 4), (n, 4), (rows, n)))
+    assert gemm._f32_ok(x, w, out) is want

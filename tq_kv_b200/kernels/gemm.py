@@ -265,10 +265,15 @@ def gemv_rows(x, w, out, bias=None, accumulate=False, swiglu=False, activation=e
     return out
 
 
+F32_TILE_MAX_COLUMNS = 64 * 65535          # column tiles of 64 gate and 64 up columns (128 of a plain product) in a grid
+
+
 def _f32_ok(x, w, out) -> bool:
-    """What csrc/gemm_f32.cu takes: float32 throughout, 16-byte pieces along K, rows that do not overlap."""
+    """What csrc/gemm_f32.cu takes: float32 throughout, 16-byte pieces along K, rows that do not overlap, and with more
+    rows than the row kernel's no more columns than a grid has tiles for."""
     K = x.shape[1]
-    return (x.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32 and K % 4 == 0
+    return ((x.shape[0] <= F32_ROW_KERNEL_MAX_ROWS or out.shape[1] <= F32_TILE_MAX_COLUMNS)
+            and x.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32 and K % 4 == 0
             and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and (x.shape[0] == 1 or (x.stride(0) >= K and out.stride(0) >= out.shape[1])) and w.stride(0) >= K)
 
