@@ -7,7 +7,7 @@ import os
 import pytest
 import torch
 
-from tq_kv_b200.kernels import gemm
+from tq_kv_b200.kernels import gemm, scan
 
 
 def _w(n, k):
@@ -70,3 +70,13 @@ def test_parts_say_that_their_weights_are_settled_and_nobody_else_is_taken_to():
 def test_float32_products_with_more_columns_than_a_grid_has_tiles_for(rows, n, want):
     x, w, out = (torch.empty(s, device="meta") for s in ((rows, 4), (n, 4), (rows, n)))
     assert gemm._f32_ok(x, w, out) is want
+
+
+@pytest.mark.parametrize("mode, silu, tokens, seqs, width, want", [
+    (scan.SCAN_DELTA, False, 8, 1, 256, True), (scan.SCAN_DELTA, False, 15, 1, 128, False), (scan.SCAN_DELTA, False, 16, 1, 128, True),
+    (scan.SCAN_DELTA, False, 47, 1, 64, False), (scan.SCAN_DELTA, False, 191, 1, 32, False), (scan.SCAN_DELTA, False, 192, 1, 32, True),
+    (scan.SCAN_DECAY, True, 31, 1, 128, False), (scan.SCAN_DECAY, True, 64, 2, 128, True), (scan.SCAN_DECAY, False, 40, 1, 128, False),
+    (scan.SCAN_GATED, False, 3000, 1, 128, True), (scan.SCAN_GATED, False, 90, 2, 128, False), (scan.SCAN_GATED, False, 90, 1, 32, False),
+    (scan.SCAN_GATED_DELTA, False, 48, 1, 64, True), (scan.SCAN_GATED_DELTA, False, 200, 1, 32, False)])
+def test_how_long_a_step_goes_eight_tokens_at_a_time(mode, silu, tokens, seqs, width, want):
+    assert scan._long_enough(mode, silu, tokens, seqs, width) is want

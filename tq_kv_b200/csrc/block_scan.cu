@@ -553,7 +553,7 @@ static long long bs_piece(int mode, int n_tokens, int n_seqs, int H, int d) {
     return (all + pieces - 1) / pieces;
 }
 
-// The line between the two scans.  Token by token, a step costs its longest sequence 210 to 350 ns a token however few
+// The line between the two scans (and how long a step must be: kernels/scan.py).  Token by token, a step costs its longest sequence 210 to 350 ns a token however few
 // columns (of the states of all heads and sequences) there are; with many columns both are bound by the SMs, and this one
 // has its records to make as well.  Measured with 128 x 128 states, one at a time / eight at a time, in us: 3,000 tokens of
 // 16 heads (2,048 columns) 1,083 / 584 (delta rule), 719 / 337 (one decay); of 32 heads (4,096 columns) 1,604 / 880, 983 /

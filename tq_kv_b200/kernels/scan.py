@@ -12,8 +12,29 @@ SCAN_DECAY, SCAN_DELTA, SCAN_GATED, SCAN_GATED_DELTA = 0, 1, 2, 3
 MAX_KEY_WIDTH = 256
 
 
-def _records(mode: int, n_tokens: int, n_seqs: int, heads: int, key_dim: int, value_dim: int, device) -> Optional[torch.Tensor]:
-    """Scratch of the scan that goes eight tokens at a time (csrc/block_scan.cu), None where the other kernel runs."""
+def _long_enough(mode: int, silu: bool, n_tokens: int, n_seqs: int, key_dim: int) -> bool:
+    """Whether a step's sequences are long enough, on average, for the scan that goes eight tokens at a time: it has its
+    records to make, 3 to 6 us that short steps do not earn back.  Measured on one sequence, 512 to 4,096 columns, in us,
+    token by token / eight at a time; delta rule: rows of 256, 8 tokens 26 / 19 to 36 / 30; 128, 16 tokens 19 / 19 to 28 /
+    26; 64, 48 tokens 24 / 24 to 30 / 26, 32 tokens 19 / 21 to 24 / 24; 32, 128 tokens 40 / 40 to 46 / 44, 64 tokens 26 / 28.
+    Constant decay behind silu (which costs the other kernel three passes): 16 tokens 15 / 13 to 27 / 28, 32 tokens 16 / 17
+    to 33 / 32.  One decay: 48 tokens 15 / 15 to 33 / 32 and with the delta rule 18 / 17 to 42 / 40, 32 tokens 13 / 15 to 28 /
+    30; rows of 32, 96 tokens 24 / 22 to 25 / 24 and with the delta rule 28 / 30 to 30 / 32, 192 tokens 50 / 46 to 51 / 52."""
+    if mode == SCAN_DELTA:
+        least = 8 if key_dim > 128 else 16 if key_dim > 64 else 48 if key_dim > 32 else 192
+    elif mode == SCAN_DECAY and silu:
+        least = 32
+    else:
+        least = 48 if key_dim > 32 else 256 if mode == SCAN_GATED_DELTA else 96
+    return n_tokens >= least * n_seqs
+
+
+def _records(mode: int, silu: bool, n_tokens: int, n_seqs: int, heads: int, key_dim: int, value_dim: int,
+             device) -> Optional[torch.Tensor]:
+    """Scratch of the scan that goes eight tokens at a time (csrc/block_scan.cu, up to 96 MB), None where the other kernel
+    runs."""
+    if not _long_enough(mode, silu, n_tokens, int(n_seqs), key_dim):
+        return None
     n = core().tq_scan_floats(mode, n_tokens, int(n_seqs), heads, key_dim, value_dim)
     return torch.empty(n, dtype=torch.float32, device=device) if n else None
 
@@ -56,7 +77,7 @@ def linear_scan(proj: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tenso
     u = a = rec = None
     ld_w = ld_u = 0
     if not single_tokens:
-        rec = _records(SCAN_DECAY if decay_logit is None else SCAN_DELTA, T, n_seqs, heads, d, e, proj.device)
+        rec = _records(SCAN_DECAY if decay_logit is None else SCAN_DELTA, silu, T, n_seqs, heads, d, e, proj.device)
     if decay_logit is not None:
         if decay_logit.dtype != torch.float32 or tuple(decay_logit.shape) != (T, heads * d) or decay_logit.stride(1) != 1:
             raise KernelError("linear_scan: decay_logit must be float32 [T, heads * d]")
@@ -186,7 +207,7 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scalars: torch
     need_contiguous(cu_seqlens=cu_seqlens, slots=slots, skip=skip)
     rec = None
     if not single_tokens:
-        rec = _records(SCAN_GATED_DELTA if delta else SCAN_GATED, T, n_seqs, heads, d, e, q.device)
+        rec = _records(SCAN_GATED_DELTA if delta else SCAN_GATED, False, T, n_seqs, heads, d, e, q.device)
     check(core().tq_gated_scan(int(bool(delta)), ptr(q), ptr(k), ptr(v), q.stride(0), ptr(scalars), ptr(skip),
                                heads // qk_heads, ptr(rec), ptr(state), state.stride(0), ptr(cu_seqlens), ptr(slots),
                                int(n_seqs), T, int(single_tokens), ptr(out), out.stride(0), heads, d, e, stream()),
