@@ -31,8 +31,10 @@ def _w(n, k):
     # a 55 MB gated product stays, a 90 MB one does not
     (8, 2 * 8960, 1536, True, True, False, False),
     (8, 2 * 11008, 2048, True, True, False, True),
-    # from 9 rows on gated products leave it at any size
-    (9, 2 * 4864, 896, True, True, False, True),
+    # from 9 rows on gated products leave it from 40 MB
+    (9, 2 * 4864, 896, True, True, False, False),
+    (16, 2 * 8192, 1024, True, True, False, False),
+    (9, 2 * 10240, 1024, True, True, False, True),
     (16, 2 * 5632, 2048, True, True, False, True),
     # over 16 rows, or with K no multiple of 32, only the tcgen05 kernel can
     (17, 896, 896, False, False, True, True),

@@ -76,7 +76,8 @@ SKINNY_MAX_ROWS = 64
 # Weights from which a decode product of up to 16 rows runs on the tcgen05 kernel (see _tc_takes)
 TC_DECODE_MIN_WEIGHT_BYTES = 24 << 20      # the product after a pending norm
 TC_DECODE_MIN_GATED_BYTES = 64 << 20       # gated products
-TC_DECODE_GATED_ROWS = 8                   # ... and these from 9 rows on at any size
+TC_DECODE_GATED_ROWS = 8                   # ... and from 9 rows on from this size
+TC_DECODE_MIN_GATED_BYTES_ROWS = 40 << 20
 TC_DECODE_MIN_ADDED_BYTES = 4 << 20        # float32 results of given rows, which leave as shares of K
 TC_DECODE_ADDED_ROWS = 8                   # ... and these from 9 rows on at any size
 
@@ -87,7 +88,9 @@ def _tc_takes(rows: int, w: torch.Tensor, swiglu: bool, after_norm: bool, float3
     size, with limits that were measured (each product alone in a replayed graph, and the whole decode step
     of the 7B and 0.5B shapes): the product after a pending norm from 24 MB on (below it the mma.sync kernel
     with the norm folded in wins: 6 MB q|k|v 4.4 against 3.8 + a norm kernel); gated products from 64 MB on
-    (55 MB at 8 rows: 12.8 against 14.3 us; 90 MB: 21.0 against 20.1); float32 results of rows that are
+    (55 MB at 8 rows: 12.8 against 14.3 us; 90 MB: 21.0 against 20.1), from 9 rows on from 40 MB (behind a norm
+    kernel, at 9 / 16 rows: 17 MB 8.9 against 10.0 / 9.0 against 10.7, 34 MB 14.3 against 14.5 / 14.9 against 16.6,
+    42 MB with K = 1,024 15.2 against 13.5 / 16.1 against 14.4, 46 MB 20.0 against 16.4 / 21.1 against 17.3); float32 results of rows that are
     given, which the tcgen05 kernel cuts into shares of K that meet in the L2, from 4 MB on and from 9 rows on
     at any size (9 MB with K = 4,864 at 8 rows: 6.1 against 4.5 us, at 16 rows 8.6 against 4.8; 5 MB with
     K = 1,536: 4.5 against 3.2; 1.6 MB at 8 rows: 2.9 against 2.7, a tie left where it was)."""
@@ -95,7 +98,7 @@ def _tc_takes(rows: int, w: torch.Tensor, swiglu: bool, after_norm: bool, float3
         return True
     size = w.numel() * 2
     if swiglu:
-        return size >= TC_DECODE_MIN_GATED_BYTES or rows > TC_DECODE_GATED_ROWS
+        return size >= (TC_DECODE_MIN_GATED_BYTES_ROWS if rows > TC_DECODE_GATED_ROWS else TC_DECODE_MIN_GATED_BYTES)
     if after_norm or not float32_out:
         return size >= TC_DECODE_MIN_WEIGHT_BYTES
     return size >= TC_DECODE_MIN_ADDED_BYTES or rows > TC_DECODE_ADDED_ROWS
