@@ -544,9 +544,10 @@ static int dg_launch(const CUtensorMap& mw, const CUtensorMap& mx, const float* 
                                     stream);
     // split K while the grid is small and the shares stay long.  Measured best on the 7B shapes: up to 4
     // blocks and about 64 blocks in all for batches over 16 rows, up to 8 and a full GPU for smaller ones.
-    // Gated products of short rows do with 64 blocks as well (16 rows, in us, a full GPU / 64 blocks: 5,632 x 2,048 17.0 /
-    // 15.6, 8,960 x 1,536 16.2 / 14.6, 4,864 x 896 11.1 / 9.3, 2,816 x 2,048 15.0 / 11.8; 5,504 x 4,096 23.6 / 25.4).
-    const bool few = M > 16 || (SWIGLU && K <= 3072);
+    // Gated products of short rows do with 64 blocks as well (a full GPU / 64 blocks, in us, 9 and 16 rows: 5,632 x 2,048 15.7 /
+    // 15.2 and 16.9 / 15.8, 8,960 x 1,536 15.3 / 14.3 and 16.8 / 15.1; longer ones do not: 6,912 x 2,560 18.4 / 19.1 and 19.9 /
+    // 19.6, 5,504 x 3,072 18.6 / 20.9 and 19.9 / 21.9, and 8,192 x 3,072 at 1 row 21.3 / 23.0, at 8 22.3 / 23.5).
+    const bool few = M > 16 || (SWIGLU && K <= 2048);
     const int max_ranks = M > 16 ? 4 : 8, want_blocks = few ? 64 : tq_sm_count();
     int ranks = 1;
     while (ranks < max_ranks && tiles * ranks < want_blocks && k_total / (ranks * 2) >= 4) ranks *= 2;
