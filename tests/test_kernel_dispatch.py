@@ -82,3 +82,13 @@ def test_float32_products_with_more_columns_than_a_grid_has_tiles_for(rows, n, w
     (scan.SCAN_GATED_DELTA, False, 48, 1, 64, True), (scan.SCAN_GATED_DELTA, False, 200, 1, 32, False)])
 def test_how_long_a_step_goes_eight_tokens_at_a_time(mode, silu, tokens, seqs, width, want):
     assert scan._long_enough(mode, silu, tokens, seqs, width) is want
+
+
+@pytest.mark.parametrize("use", [True, False])
+def test_the_tcgen05_switch_leaves_the_row_kernel_alone(use, monkeypatch):
+    """It runs on FMA units."""
+    monkeypatch.setattr(gemm, "USE_TCGEN05", use)
+    ran = []
+    monkeypatch.setattr(gemm, "row_gemm", lambda x, w, out, *a: ran.append(w.shape) or out)
+    gemm.linear(torch.empty(1, 2048, dtype=torch.bfloat16, device="meta"), _w(10304, 2048))
+    assert ran == [(10304, 2048)]

@@ -111,14 +111,14 @@ ROW_GEMM_HEAD_COLUMNS = 16384              # ... with so many columns
 
 
 def _row_takes(rows: int, w: torch.Tensor, swiglu: bool) -> bool:
-    """Which bfloat16 products of one row run on the FMA row kernel (csrc/row_gemm.cu), by the weight's size.  Measured in
-    whole passes of prompts and 24 decoded tokens, in ms, none / these / these without gated ones / without heads: 7B 72.4
-    / 71.0 / 70.7 / 71.6, zodosun-2k 20.2 / 18.7 / 19.4 / 18.9, rirudra-2k 9.73 / 8.72 / 9.00 / 9.05 (weights of 17 to
-    46 MB a product there, 26 and 33 MB in the 7B shape); given up to 24 MB only: 72.1 / 20.1 / 9.70.  Alone in replayed
-    graphs, in us: 9 MB 4.2 on the other kernel / 4.4 here, 23 MB 7.1 / 6.5, 26 MB 7.1 / 6.4, gated 17 MB 5.0 / 5.4,
-    gated 46 MB 11.7 / 10.3, 136 MB 23.9 / 23.6 (and in the 7B shape's step slower: its 3,584 long columns), a head of
-    272 MB 48.8 / 41.5.  With the norm made by the row kernel itself passes were slower (0.5B 15.9 -> 16.8 ms), two rows
-    gain little (a head 49.1 / 46.5) or lose (26 MB 7.0 / 8.7)."""
+    """Which bfloat16 products of one row run on the FMA row kernel (csrc/row_gemm.cu), by the weight's size.  In replayed
+    graphs of the same product with other weights, in us, the other kernel / here: 17 MB 8.2 / 4.8 (K = 2,048 and 1,024), 23
+    MB 7.1 / 6.5, 25 MB 9.4 / 6.1, 33 MB 10.9 / 7.5 (K = 4,096) and 10.3 / 7.6 (K = 8,192), 35 MB 10.7 / 8.9, 52 MB 13.4 / 11.2;
+    gated 46 MB 11.7 / 10.3, 50 MB 15.3 / 10.7, 55 MB 12.8 / 10.8, 59 MB 15.8 / 12.0, 63 MB 22.2 / 13.3; heads of 33 MB 9.0 /
+    7.6, 77 MB 18.9 / 15.4, 272 MB 48.8 / 41.5.  Outside: 9 MB 4.2 / 4.4, gated 17 MB 5.0 / 5.4, 136 MB 23.9 / 23.6 (and in
+    the 7B shape's step slower: its 3,584 long columns).  Whole passes of a prompt and 24 decoded tokens, in ms, without /
+    with these: 7B 72.4 / 71.0, zodosun-2k 20.2 / 18.7, rirudra-2k 9.73 / 8.72.  With the norm made by the row kernel itself
+    passes were slower (0.5B 15.9 -> 16.8 ms), two rows gain little (a head 49.1 / 46.5) or lose (26 MB 7.0 / 8.7)."""
     if rows != 1:
         return False
     size = w.numel() * 2
@@ -334,7 +334,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = N
             return out
         x = pending.materialize()
 
-    if (_row_takes(M, w, bool(swiglu)) and USE_TCGEN05 and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K % 8 == 0
+    if (_row_takes(M, w, bool(swiglu)) and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K % 8 == 0
             and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and out.dtype in (torch.float32, torch.bfloat16) and (not accumulate or out.dtype == torch.float32)):
         return row_gemm(x, w, out, bias, accumulate, swiglu, activation, w_settled)
