@@ -43,3 +43,14 @@ def within(out, want, dtype):
 def test_a_result_that_starts_between_two_pairs(hd, dtype, shift):
     out, want = run(hd, 3, [400, 5, 130], dtype, shift=shift)
     within(out, want, dtype)
+
+
+@pytest.mark.parametrize("hd,n_splits", [(64, 64), (128, 64), (128, 65), (200, 33), (256, 32), (256, 33), (256, 64), (512, 16),
+                                         (512, 17), (512, 40), (512, 64)])
+@pytest.mark.parametrize("with_sink", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_more_splits_than_are_asked_for_ahead(hd, n_splits, with_sink, dtype):
+    """Beside a long sequence whose splits all hold keys, short ones whose last splits hold none."""
+    sink = torch.tensor([0.5, -1.0, 3.0], device=DEV) if with_sink else None
+    out, want = run(hd, n_splits, [4500, 70, 0, 900], dtype, sink=sink)
+    within(out, want, dtype)

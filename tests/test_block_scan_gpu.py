@@ -119,8 +119,12 @@ def test_against_float64(mode, lens, H, G, d, e):
 def test_a_step_cut_into_pieces(mode):
     """More records than one piece takes: the state waits in its slot between the pieces."""
     from tq_kv_b200 import kernels
-    H, d, lens = 16, 128, [2500, 700]
-    assert kernels._lib.core().tq_scan_floats(1 if mode == "delta" else 2, sum(lens), 2, H, d, d) * 4 <= 100 << 20
+    H, d, lens = 16, 128, [2500, 700] if mode == "delta" else [3600, 2400]
+    floats = kernels._lib.core().tq_scan_floats(1 if mode == "delta" else 2, sum(lens), 2, H, d, d)
+    record = (4 if mode == "delta" else 2) * 8 * d + 2 * d + (16 if mode == "delta" else 8) * 8
+    all_records = sum(-(-n // 8) for n in lens)
+    assert floats * 4 <= 96 << 20 and floats < all_records * H * record          # two pieces
+    assert floats // (H * record) < -(-lens[0] // 8)                              # the second sequence starts in the second
     p = make(mode, lens, H, H, d, d, seed=3)
     out, state = run(mode, p, lens, [1, 3], H, H, d, d)
     want, want_state = exact(mode, p, lens, [1, 3], H, H, d, d)

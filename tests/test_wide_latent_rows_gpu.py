@@ -76,25 +76,25 @@ def test_against_float64_and_the_general_kernel(hd, heads, n_splits, window, wit
 
 
 def test_a_weight_keeps_its_24_bits():
-    """Two equal keys and a third far below: the third's weight, 2^-14 of the others, moves the mean of values that
-    cancel, and would be lost in a weight rounded to bfloat16."""
+    """Two weights of about 0.71 that differ by 2^-12 of themselves, with values of 1 and -1: the mean is their small
+    difference.  Weights of one bfloat16 part would be 20 times off, of two parts 1.2 % (computed on the CPU); of three the
+    result's own rounding (2^-9) is what is left, and the exponential's, 1e-7 of the weights or 5e-4 of the difference."""
     from tq_kv_b200 import kernels
     hd = 256
     rows = torch.zeros(1, 1, 64, hd, device=DEV)
-    rows[0, 0, 0, 0] = rows[0, 0, 1, 0] = 1.0
-    rows[0, 0, 0, 1], rows[0, 0, 1, 1], rows[0, 0, 2, 1] = 1.0, -1.0, 1.0
-    rows[0, 0, 2, 0] = 1.0 - 14 * math.log(2.0) / 16.0
+    rows[0, 0, :3, 0] = torch.tensor([3.125, 0.375, 0.375 - 2.0 ** -9])
+    rows[0, 0, 1, 1], rows[0, 0, 2, 1] = 1.0, -1.0
     pages = rows.to(torch.bfloat16)
+    assert torch.equal(pages.float(), rows)
     q = torch.zeros(1, hd, device=DEV, dtype=torch.bfloat16)
-    q[0, 0] = 16.0
+    q[0, 0] = 0.125
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
     out = torch.empty_like(q)
     kernels.attention(q, out, n_heads=1, n_kv_heads=1, head_dim=hd, tok_pos=i32([2]), tok_seq=i32([0]), cu_seqlens=i32([0, 1]),
                       start_pos=i32([2]), window=None, scale=1.0, k_pages=pages, v_pages=pages, block_table=i32([[0]]),
                       table_width=1)
     r = pages[0, 0, :3].double()
-    w = (16.0 * r[:, 0]).softmax(0)
-    want = w @ r
+    want = (0.125 * r[:, 0]).softmax(0) @ r
     assert float((out[0].double() - want).abs()[1]) <= 2.0 ** -8 * float(want[1].abs())
 
 
