@@ -18,15 +18,18 @@
 //                                              E_ij = D_ij + sum_{j<m<=i} C_im F_mj,         D_ij = q_i . (w_{j+1..i} * x_j)
 //   S' = diag(w_{0..7}) S + sum_j N_j r_j + X_j v_j,      N_j = w_{j+1..7} * n_j,   X_j = w_{j+1..7} * x_j
 //
-// so that all 16 products with the state are independent of one another and the chain is one step in eight.  Every
-// decay enters as a product of decays, never as a quotient: nothing overflows however fast a channel fades.  All float32.
+// so that all 16 products with the state are independent of one another and the chain is one step in eight.  All float32.
+// Decays enter as products: nothing overflows however fast a head fades.  Only the sums A to D of SCAN_DELTA, whose decays
+// differ by channel, take the decays between two tokens as a quotient of two products; that is sound because eight of its
+// decays are at least 0.008 (block_prepare), and is not for a decay per channel without such a bound.
 //
-// block_prepare   a warp per (eight tokens, head) makes P, Q, N, X, the decays' product and the rows of F and E once
-//                 for all columns, as one record; it also makes w, u and a * u from their logits and applies silu.
+// block_prepare   a block per (eight tokens, head), a thread a key channel, makes P, Q, N, X, the decays' product and the
+//                 rows of F and E once for all columns, as one record; it also makes w, u and a * u from their logits
+//                 and applies silu.
 //                 The records of a step start at each sequence's first token; the last one of a sequence is filled up
 //                 with tokens that change nothing (w = 1, all vectors 0).
-// block_scan      a block owns some columns of one head of one sequence and walks the records in order, every thread 8
-//                 keys x RC columns of the state in registers, the records three stages deep in shared memory
+// block_scan      a block owns some columns of one head of one sequence and walks the records in order, every thread 4
+//                 keys (8 of rows over 128) x RC columns of the state in registers, the records three stages deep in shared memory
 //                 (cp.async).  The sums over the KG lanes that share a column are made by trading halves of the values,
 //                 so that each lane ends with the few sums that it completes (F v, E v) and hands on.
 //
@@ -528,8 +531,10 @@ static int launch_block_scan(const ScanArgs& a, int n_seqs, int rec0, int rec1, 
 }
 
 // Which form.  A thread holds four keys (eight of rows over 128), so that every load brings different entries to all 32
-// lanes; 8 or 16 columns a block.  Measured with 128 x 128 states, 3,000 tokens of one sequence, in us (columns a block x
-// threads; delta rule / one decay): 16 heads: 8 x 128 488 / 331, 16 x 256 490 / 346, 16 x 128 (eight keys a thread) 540 /
+// lanes; a block of 128 threads with two columns each (8 columns of rows over 64, 16 and 32 of shorter ones) while there are
+// at most two such blocks an SM, else of 256 threads with four each (32, 64 and 128 columns).  Measured with 128 x 128
+// states, 3,000 tokens of one sequence, in us, before the sums were compensated (columns a block x threads; delta rule /
+// one decay): 16 heads: 8 x 128 488 / 331, 16 x 256 490 / 346, 16 x 128 (eight keys a thread) 540 /
 // 352; 32 heads: 8 x 128 763 / 487, 16 x 128 702 / 568, 32 x 256 707 / 447.
 template <bool DELTA, bool APART, int DP>
 static int pick_block_scan(const ScanArgs& a, int n_seqs, int rec0, int rec1, int silu_v, const float* rec, cudaStream_t stream) {
