@@ -215,9 +215,23 @@ __device__ __forceinline__ void tc_epilogue_item(uint32_t t_row, unsigned char* 
     }
 }
 
+// Tile t of the pair form -> its place: bands of T2_BAND rows of tiles, column by column within a band, so that the 74
+// pairs work on a patch of about 16 x 5 tiles at a time.  Column by column over all rows a round of many rows reads all of A
+// for one or two columns of tiles: 15,500 rows (61 rows of tiles, 110 MB of A with K = 3,584) came from DRAM once a round,
+// and under the power cap that costs clocks.  Measured, the products of a 7B layer in turn at the power cap, TFLOP/s, all
+// rows / bands of 4 / 8 / 12 / 16 / 24: 15,500 rows 1,125 / 1,245 / 1,284 / 1,293 / 1,300 / 1,287, 7,400 rows 1,283 / 1,256 /
+// 1,287 / 1,290 / 1,306 / 1,290.  Up to 4,096 rows one band holds them all, as before.
+#define T2_BAND 16
+__device__ __forceinline__ void tc_place(int t, int tiles_m, int tiles_n, int& tm, int& tn) {
+    const int first = t / (T2_BAND * tiles_n) * T2_BAND, r = t - first * tiles_n;
+    const int rows = min(T2_BAND, tiles_m - first);
+    tn = r / rows;
+    tm = first + r - tn * rows;
+}
+
 // ---- the kernel -------------------------------------------------------------------
 // Persistent: one block per SM walks the output tiles t = blockIdx.x, + gridDim.x, ...
-// (tiles that share a B tile are neighbours, so they meet in L2).  Two
+// (tiles that share a B tile are neighbours, so they meet in L2; the pair form: tc_place).  Two
 // accumulators of 256 TMEM columns alternate, so the MMAs of a tile overlap
 // the epilogue of the tile before.  b_rows_second: SwiGLU only — row offset
 // of the up rows in B (the number of outputs).
@@ -505,8 +519,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             for (int w = pair; w < n_items && ok; w += n_pairs) {
                 int t, k_lo, k_iters, part;
                 item(w, t, k_lo, k_iters, part);
-                const int m0 = (t % tiles_m) * 2 * TC_BM + (int)rank * TC_BM;
-                const int n0 = (t / tiles_m) * OUT_COLS;
+                int tm, tn;
+                tc_place(t, tiles_m, tiles_n, tm, tn);
+                const int m0 = tm * 2 * TC_BM + (int)rank * TC_BM;
+                const int n0 = tn * OUT_COLS;
                 const int b_row = TC_GATED(EPI) ? (rank == 0 ? n0 : b_rows_second + n0) : n0 + (int)rank * (TC_BN / 2);
                 for (int i = 0; i < k_iters; ++i, ++it) {
                     const int s = it % T2_STAGES;
@@ -557,7 +573,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         for (int w = pair; w < n_items && ok; w += n_pairs, ++local) {
             int t, k_lo, k_iters, part;
             item(w, t, k_lo, k_iters, part);
-            const int m0 = (t % tiles_m) * 2 * TC_BM + (int)rank * TC_BM, n0 = (t / tiles_m) * OUT_COLS;
+            int tm, tn;
+            tc_place(t, tiles_m, tiles_n, tm, tn);
+            const int m0 = tm * 2 * TC_BM + (int)rank * TC_BM, n0 = tn * OUT_COLS;
             const uint32_t buf = local & 1;
             if (!mbar_wait(smem_u32(&acc_full[buf]), (local >> 1) & 1, true)) { *failed = 1; ok = false; break; }
             tc_fence_after();
