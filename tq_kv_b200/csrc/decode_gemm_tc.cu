@@ -4,8 +4,8 @@
 // accumulator D[128 weight rows x batch] sits in TMEM with one weight row per
 // lane.  Y[M,N] = X[M,K] · W[N,K]^T.
 //
-// A block owns 128 output columns (64 with SwiGLU: 64 gate rows and the 64 up
-// rows of the same outputs share a tile) and a share of K; W and X tiles come
+// A block owns 128 output columns (64 of a gated product, which comes here with a norm folded in only: 64 gate rows and the
+// 64 up rows of the same outputs share a tile) and a share of K; W and X tiles come
 // in by TMA through a 4-stage mbarrier pipeline (16 KB of W per stage; two
 // blocks fit an SM, so ~128 KB of weights are in flight per SM and one
 // block's epilogue runs under the other's loads).  Where 128-row tiles alone give
@@ -85,7 +85,7 @@ __device__ __forceinline__ void dg_ld32(uint32_t taddr, float* v) {
 // cluster's exchange, where every output is scaled by 1 / sqrt(mean(h^2) + eps) of its batch row.  So the norm
 // needs no kernel and no trip through memory of its own.
 // The gate's activation of a gated product (TQ_ACT_*), or TQ_ACT_SQUARE_RELU on a plain one with a bfloat16 result
-// (its K is never cut into independent shares): the exported functions set it from their `swiglu` argument (1 or 2:
+// (its K is never cut into independent shares): the exported functions set it from their `swiglu` or `gate` argument (1 or 2:
 // gated; 3: plain, squared relu; 0: plain) right before they launch, on the launching thread.
 static thread_local int dg_gate_act = TQ_ACT_SILU;
 #define DG_NORM_ROWS 16
@@ -529,63 +529,52 @@ static int dg_reduce_shares(int N, int K) {
 // can then ask for accumulation and save the clearing.
 TQ_API int tq_decode_gemm_tc_adds_shares(int N, int K) { return dg_reduce_shares(N, K) > 1 ? 1 : 0; }
 
-template <int MP, bool SWIGLU, typename TO>
+template <int MP, typename TO>
 static int dg_launch(const CUtensorMap& mw, const CUtensorMap& mx, const float* bias, void* Y, int M, int N, int K,
                      int ldy, int accumulate, int* status, cudaStream_t stream) {
-    constexpr int OUT_COLS = SWIGLU ? DG_ROWS / 2 : DG_ROWS;
-    const int tiles = (N + OUT_COLS - 1) / OUT_COLS;
+    const int tiles = (N + DG_ROWS - 1) / DG_ROWS;
     const int k_total = (K + DG_BK - 1) / DG_BK;
     // Float32 results without gating: where the tiles do not fill the GPU's block slots (two per SM), independent
     // shares of K, as many as still run in one wave (dg_reduce_shares).  These results leave through TMA (a store for a single share that is not added to anything,
     // else a reduce-add), which costs a block far less than the exchange and the element-wise stores of the
     // cluster form below.  Y must be fit for TMA (16-byte aligned base and row stride).
-    if (!SWIGLU && sizeof(TO) == 4 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (ldy & 3) == 0)
+    if (sizeof(TO) == 4 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (ldy & 3) == 0)
         return dg_launch_reduce<MP>(mw, mx, bias, (float*)Y, M, N, K, ldy, accumulate, status, dg_reduce_shares(N, K),
                                     stream);
     // split K while the grid is small and the shares stay long.  Measured best on the 7B shapes: up to 4
     // blocks and about 64 blocks in all for batches over 16 rows, up to 8 and a full GPU for smaller ones.
-    // Gated products of short rows do with 64 blocks as well (a full GPU / 64 blocks, in us, 9 and 16 rows: 5,632 x 2,048 15.7 /
-    // 15.2 and 16.9 / 15.8, 8,960 x 1,536 15.3 / 14.3 and 16.8 / 15.1; longer ones do not: 6,912 x 2,560 18.4 / 19.1 and 19.9 /
-    // 19.6, 5,504 x 3,072 18.6 / 20.9 and 19.9 / 21.9, and 8,192 x 3,072 at 1 row 21.3 / 23.0, at 8 22.3 / 23.5).
-    const bool few = M > 16 || (SWIGLU && K <= 2048);
-    const int max_ranks = M > 16 ? 4 : 8, want_blocks = few ? 64 : tq_sm_count();
+    const int max_ranks = M > 16 ? 4 : 8, want_blocks = M > 16 ? 64 : tq_sm_count();
     int ranks = 1;
     while (ranks < max_ranks && tiles * ranks < want_blocks && k_total / (ranks * 2) >= 4) ranks *= 2;
-    return dg_launch_s<MP, SWIGLU, TO, 4>(mw, mx, bias, Y, M, N, K, ldy, accumulate, status, ranks, stream);
+    return dg_launch_s<MP, false, TO, 4>(mw, mx, bias, Y, M, N, K, ldy, accumulate, status, ranks, stream);
 }
 
-// X [M <= 64, K] and W [N, K] (or [2N, K] with swiglu) bfloat16, row strides
+// X [M <= 64, K] and W [N, K] bfloat16, row strides
 // ldx / ldw elements (multiples of 8, bases 16-byte aligned); Y [M, N]
-// float32 or bfloat16 (accumulate needs float32).
+// float32 or bfloat16 (accumulate needs float32).  gate: 0, or TQ_ACT_SQUARE_RELU with a bfloat16 result (gated products:
+// decode_pair_tc.cu, and below with a norm folded in).
 TQ_API int tq_decode_gemm_tc(const void* X, const void* W, const float* bias, void* Y, int y_dtype, int M, int N, int K,
-                             int ldx, int ldw, int ldy, int accumulate, int swiglu, int* status, cudaStream_t stream) {
+                             int ldx, int ldw, int ldy, int accumulate, int gate, int* status, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (M > 64 || K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7)) return (int)cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(X) & 15) || (reinterpret_cast<uintptr_t>(W) & 15))
         return (int)cudaErrorInvalidValue;
     if (accumulate && y_dtype != TQ_F32) return (int)cudaErrorInvalidValue;
-    if (swiglu < 0 || swiglu > TQ_ACT_SQUARE_RELU || (swiglu == TQ_ACT_SQUARE_RELU && y_dtype != TQ_BF16))
-        return (int)cudaErrorInvalidValue;
-    dg_gate_act = swiglu ? swiglu : TQ_ACT_SILU;
-    if (swiglu == TQ_ACT_SQUARE_RELU) swiglu = 0;
+    if (gate != 0 && (gate != TQ_ACT_SQUARE_RELU || y_dtype != TQ_BF16)) return (int)cudaErrorInvalidValue;
+    dg_gate_act = gate ? gate : TQ_ACT_SILU;
     const int mp = M <= 32 ? 32 : 64;
     CUtensorMap mw, mx;
-    int st = dg_make_map(&mw, W, swiglu ? 2ull * N : (uint64_t)N, (uint64_t)K, (uint64_t)ldw,
-                         swiglu ? DG_ROWS / 2 : DG_ROWS);
+    int st = dg_make_map(&mw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, DG_ROWS);
     if (st) return st;
     st = dg_make_map(&mx, X, (uint64_t)M, (uint64_t)K, (uint64_t)ldx, mp);
     if (st) return st;
-#define TQ_DG(MP, S, T) return dg_launch<MP, S, T>(mw, mx, bias, Y, M, N, K, ldy, accumulate, status, stream)
+#define TQ_DG(MP, T) return dg_launch<MP, T>(mw, mx, bias, Y, M, N, K, ldy, accumulate, status, stream)
     if (mp == 32) {
-        if (swiglu && y_dtype == TQ_BF16) TQ_DG(32, true, bf16);
-        if (swiglu && y_dtype == TQ_F32) TQ_DG(32, true, float);
-        if (!swiglu && y_dtype == TQ_BF16) TQ_DG(32, false, bf16);
-        if (!swiglu && y_dtype == TQ_F32) TQ_DG(32, false, float);
+        if (y_dtype == TQ_BF16) TQ_DG(32, bf16);
+        if (y_dtype == TQ_F32) TQ_DG(32, float);
     } else {
-        if (swiglu && y_dtype == TQ_BF16) TQ_DG(64, true, bf16);
-        if (swiglu && y_dtype == TQ_F32) TQ_DG(64, true, float);
-        if (!swiglu && y_dtype == TQ_BF16) TQ_DG(64, false, bf16);
-        if (!swiglu && y_dtype == TQ_F32) TQ_DG(64, false, float);
+        if (y_dtype == TQ_BF16) TQ_DG(64, bf16);
+        if (y_dtype == TQ_F32) TQ_DG(64, float);
     }
 #undef TQ_DG
     return (int)cudaErrorInvalidValue;

@@ -13,7 +13,8 @@
 //   routed_gate_up:  act[t*top + s, i] = silu(x[t] . gate[e][i]) * (x[t] . up[e][i])
 //   routed_down:     y[t, c] (+)= 1/top * sum_s act[t*top + s] . down[e_s][c]     (the experts in the table's order)
 // Many tokens: the rows are sorted by expert so that each expert's rows form whole tiles of a matrix product
-// (routed_plan / routed_gather / routed_combine below; the products themselves are csrc/gemm_tc.cu's).
+// (routed_plan / routed_gather / routed_combine below; the products themselves are csrc/decode_pair_tc.cu's up to 64 tokens
+// and csrc/gemm_tc.cu's beyond).
 #include "common.cuh"
 
 // ---- choice: experts of each token from a table indexed by the token id ------------------------------------------
@@ -290,11 +291,12 @@ TQ_API int tq_routed_experts_rows(const void* x, int x_dtype, int ldx, const voi
 // One block plans the step: it counts the (token, expert) pairs of each expert, gives each expert a run of whole
 // tiles of `tile` rows in a sorted buffer (experts in index order), tells every tile which rows of the stacked
 // weights it multiplies with (tile_b_up / tile_b_down: the expert's first row there; -1 for tiles past the last
-// used one) and gives each pair its row in the buffer (pos).  Which of an expert's rows a pair gets depends on
+// used one), how many of its rows are used (tile_rows, or null) and gives each pair its row in the buffer (pos).  Which of an expert's rows a pair gets depends on
 // the order the threads arrive in; a row's result does not depend on where in a tile it lies.
 __global__ void __launch_bounds__(1024)
 routed_plan_kernel(const int* __restrict__ choice, int n_pairs, int n_experts, int tile, int up_rows, int down_rows,
-                   int max_tiles, int* __restrict__ pos, int* __restrict__ tile_b_up, int* __restrict__ tile_b_down) {
+                   int max_tiles, int* __restrict__ pos, int* __restrict__ tile_b_up, int* __restrict__ tile_b_down,
+                   int* __restrict__ tile_rows) {
     extern __shared__ int plan_sh[];         // counts [E], first row [E], cursor [E]
     int* counts = plan_sh;
     int* first = plan_sh + n_experts;
@@ -313,6 +315,7 @@ routed_plan_kernel(const int* __restrict__ choice, int n_pairs, int n_experts, i
             for (int i = 0; i < n && t < max_tiles; ++i, ++t) {
                 tile_b_up[t] = e * up_rows;
                 tile_b_down[t] = e * down_rows;
+                if (tile_rows) tile_rows[t] = min(tile, counts[e] - i * tile);
             }
         }
         for (; t < max_tiles; ++t) { tile_b_up[t] = -1; tile_b_down[t] = -1; }
@@ -371,11 +374,12 @@ routed_combine_kernel(const float* __restrict__ out, const int* __restrict__ pos
     }
 }
 
-// The plan and the gather of a step.  choice [T*top]; pos [T*top], tile_b_up / tile_b_down [max_tiles] (outputs);
+// The plan and the gather of a step.  choice [T*top]; pos [T*top], tile_b_up / tile_b_down / tile_rows (or null)
+// [max_tiles] (outputs);
 // sorted [max_tiles*tile, W] bfloat16 (rows that no pair owns keep what they held: nobody reads their results).
 TQ_API int tq_routed_sort(const void* x, int ldx, const int* choice, int top, int n_tokens, int W, int n_experts,
                           int tile, int up_rows, int down_rows, int max_tiles, int* pos, int* tile_b_up,
-                          int* tile_b_down, void* sorted, cudaStream_t stream) {
+                          int* tile_b_down, int* tile_rows, void* sorted, cudaStream_t stream) {
     const int n_pairs = n_tokens * top;
     if (n_pairs <= 0) return 0;
     if (W % 8 || ldx % 8 || n_experts < 1 || n_experts > 4096 || tile < 1 || !aligned16(x) || !aligned16(sorted))
@@ -383,7 +387,7 @@ TQ_API int tq_routed_sort(const void* x, int ldx, const int* choice, int top, in
     if (max_tiles < (n_pairs + tile - 1) / tile + n_experts - 1 && max_tiles < n_pairs) return (int)cudaErrorInvalidValue;
     int st = tq_launch_pdl(TQ_PDL_ELEMENTWISE, routed_plan_kernel, dim3(1), dim3(1024), (size_t)3 * n_experts * sizeof(int),
                            stream, choice, n_pairs, n_experts, tile, up_rows, down_rows, max_tiles, pos, tile_b_up,
-                           tile_b_down);
+                           tile_b_down, tile_rows);
     if (st) return st;
     return tq_launch_pdl(TQ_PDL_ELEMENTWISE, routed_gather_kernel, dim3((n_pairs + 7) / 8), dim3(256), 0, stream,
                          (const bf16*)x, ldx, (const int*)pos, top, W, n_pairs, (bf16*)sorted);

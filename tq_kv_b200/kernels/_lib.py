@@ -173,6 +173,10 @@ _SIGNATURES = {
     "tq_decode_gemm_tc_adds_shares": [c_int, c_int],
     "tq_decode_gemm_tc": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                           c_int, c_int, c_void_p, c_void_p],
+    "tq_decode_pair_tc": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                          c_int, c_void_p, c_void_p],
+    "tq_decode_pair_tc_grouped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                                  c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     "tq_flash_decode": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                         c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "tq_flash_prefill": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p,
@@ -268,7 +272,7 @@ _SIGNATURES = {
     "tq_channel_decay": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "tq_round_columns": [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p],
     "tq_routed_sort": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
-                       c_void_p, c_void_p, c_void_p, c_void_p],
+                       c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     "tq_routed_combine": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,
                           c_void_p],
     "tq_gemm_tc_grouped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,

@@ -6,6 +6,7 @@ from typing import Optional
 import torch
 
 from ._lib import KernelError, check, core, dtype_code, need_contiguous, ptr, stream, tc_status_word
+from .elementwise import ACT_SILU, ACT_SQUARE_RELU
 
 
 def table_choice(tokens: torch.Tensor, table: torch.Tensor, n_experts: int) -> torch.Tensor:
@@ -111,7 +112,8 @@ def routed_experts_rows(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.
     return y
 
 
-TILE_ROWS = 128                     # rows of a tile of the tensor-core products (csrc/gemm_tc.cu)
+TILE_ROWS = 128                     # rows of a tile of the many-row tensor-core products (csrc/gemm_tc.cu)
+FEW_TILE_ROWS = 64                  # ... and of those that stream the weights past few rows (csrc/decode_pair_tc.cu)
 
 
 def routed_tiles_ok(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, gated: bool = True) -> bool:
@@ -127,7 +129,8 @@ def routed_experts_tiles(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch
                          gated: bool = True, shared: Optional[torch.Tensor] = None,
                          shared_gate: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The same result as `routed_experts_rows` for many rows: the (token, expert) pairs are sorted by expert
-    into a buffer in which every expert owns whole tiles of 128 rows; two tensor-core products over the whole
+    into a buffer in which every expert owns whole tiles of 128 rows (up to 64 tokens: of as many rows as there are
+    tokens, in steps of 16); two tensor-core products over the whole
     buffer follow, in which each tile multiplies with its own expert's matrices (the first gates, silu(g) * u,
     in its epilogue; without a gate it squares its relu there), and a last kernel takes each token's rows back and averages them."""
     T, W = x.shape
@@ -142,22 +145,32 @@ def routed_experts_tiles(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch
     ldg = _check_shared(shared, shared_gate, y, weights)
     top = choice.shape[1]
     n_pairs = T * top
-    max_tiles = n_pairs // TILE_ROWS + E
-    rows = max_tiles * TILE_ROWS
+    few = T <= FEW_TILE_ROWS
+    tile = -(-T // 16) * 16 if few else TILE_ROWS
+    max_tiles = n_pairs // tile + E
+    rows = max_tiles * tile
     dev = x.device
-    plan = torch.empty(n_pairs + 2 * max_tiles, dtype=torch.int32, device=dev)
-    pos, tile_up, tile_down = plan[:n_pairs], plan[n_pairs:n_pairs + max_tiles], plan[n_pairs + max_tiles:]
+    plan = torch.empty(n_pairs + 3 * max_tiles, dtype=torch.int32, device=dev)
+    pos, tile_up, tile_down, tile_rows = plan.split([n_pairs, max_tiles, max_tiles, max_tiles])
     sorted_x = torch.empty((rows, W), dtype=torch.bfloat16, device=dev)
     act = torch.empty((rows, F), dtype=torch.bfloat16, device=dev)
     out = torch.empty((rows, W), dtype=torch.float32, device=dev)
     lib = core()
-    check(lib.tq_routed_sort(ptr(x), x.stride(0), ptr(choice), top, T, W, E, TILE_ROWS, F2, W, max_tiles, ptr(pos),
-                             ptr(tile_up), ptr(tile_down), ptr(sorted_x), stream()), "routed_sort", 2)
+    check(lib.tq_routed_sort(ptr(x), x.stride(0), ptr(choice), top, T, W, E, tile, F2, W, max_tiles, ptr(pos),
+                             ptr(tile_up), ptr(tile_down), ptr(tile_rows), ptr(sorted_x), stream()), "routed_sort", 2)
     status = ptr(tc_status_word(dev))
-    check(lib.tq_gemm_tc_grouped(ptr(sorted_x), ptr(w_gate_up), ptr(act), dtype_code(act), rows, F, W, W, W, F,
-                                 2 if gated else 4, E * F2, F if gated else 0, ptr(tile_up), status, stream()), "routed_gate_up")
-    check(lib.tq_gemm_tc_grouped(ptr(act), ptr(w_down), ptr(out), dtype_code(out), rows, W, F, F, F, W,
-                                 0, E * W, 0, ptr(tile_down), status, stream()), "routed_down")
+    if few:                             # (no expert has more rows than there are tokens: one tile each)
+        live = min(E, n_pairs)
+        check(lib.tq_decode_pair_tc_grouped(ptr(sorted_x), ptr(w_gate_up), ptr(act), dtype_code(act), tile, max_tiles, live, F, W, W, W, F,
+                                            ACT_SILU if gated else ACT_SQUARE_RELU, E * F2, ptr(tile_up), ptr(tile_rows),
+                                            status, stream()), "routed_gate_up")
+        check(lib.tq_decode_pair_tc_grouped(ptr(act), ptr(w_down), ptr(out), dtype_code(out), tile, max_tiles, live, W, F, F, F, W, 0,
+                                            E * W, ptr(tile_down), ptr(tile_rows), status, stream()), "routed_down")
+    else:
+        check(lib.tq_gemm_tc_grouped(ptr(sorted_x), ptr(w_gate_up), ptr(act), dtype_code(act), rows, F, W, W, W, F,
+                                     2 if gated else 4, E * F2, F if gated else 0, ptr(tile_up), status, stream()), "routed_gate_up")
+        check(lib.tq_gemm_tc_grouped(ptr(act), ptr(w_down), ptr(out), dtype_code(out), rows, W, F, F, F, W,
+                                     0, E * W, 0, ptr(tile_down), status, stream()), "routed_down")
     check(lib.tq_routed_combine(ptr(out), ptr(pos), ptr(weights), top, T, W, ptr(y), int(accumulate), ptr(shared),
                                 ptr(shared_gate), ldg, stream()), "routed_combine")
     return y

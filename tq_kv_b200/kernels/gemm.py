@@ -7,8 +7,9 @@
     limits are in `_tc_takes`): the weight-streaming mma.sync kernel of
     csrc/skinny_gemm.cu, which reads the weight once and fuses bias, SwiGLU
     gating and the float32 accumulation into the residual stream;
-  * up to 64 rows of bfloat16 otherwise: the same job on tcgen05 with swapped
-    operands, TMA-fed (csrc/decode_gemm_tc.cu);
+  * up to 64 rows of bfloat16 otherwise: the same job on tcgen05, TMA-fed
+    (csrc/decode_pair_tc.cu for gated products, see `_pair_takes`; csrc/decode_gemm_tc.cu, with
+    swapped operands, for the others);
   * up to 16 rows of anything else: the float32 row kernel of csrc/gemm.cu
     with the same epilogues;
   * many rows, bfloat16 × bfloat16: the TMA + tcgen05 kernels of
@@ -83,7 +84,8 @@ TC_DECODE_ADDED_ROWS = 8                   # ... and these from 9 rows on at any
 
 
 def _tc_takes(rows: int, w: torch.Tensor, swiglu: bool, after_norm: bool, float32_out: bool) -> bool:
-    """Which of the two decode kernels gets a bfloat16 product that both can run: True for the TMA-fed
+    """Which of the two decode kernels gets a bfloat16 product that both can run (gated: which one folds a pending norm
+    in; without one `_pair_takes` decides): True for the TMA-fed
     tcgen05 kernel, False for the mma.sync one.  Over 16 rows always the former.  Below that by the weight's
     size, with limits that were measured (each product alone in a replayed graph, and the whole decode step
     of the 7B and 0.5B shapes): the product after a pending norm from 24 MB on (below it the mma.sync kernel
@@ -125,6 +127,25 @@ def _row_takes(rows: int, w: torch.Tensor, swiglu: bool) -> bool:
     if not swiglu and w.shape[0] >= ROW_GEMM_HEAD_COLUMNS:
         return size >= ROW_GEMM_MIN_BYTES
     return (ROW_GEMM_MIN_GATED_BYTES if swiglu else ROW_GEMM_MIN_BYTES) <= size <= ROW_GEMM_MAX_BYTES
+
+
+PAIR_MIN_BYTES_ROWS = 20 << 20             # gated products of 9 to 16 rows: from this size
+PAIR_MIN_BYTES = 40 << 20                  # ... of up to 8 rows
+
+
+def _pair_takes(rows: int, w: torch.Tensor) -> bool:
+    """Which gated bfloat16 products of given rows (a norm that is not folded in) run on csrc/decode_pair_tc.cu, by the
+    weight's size: all of more than 16 rows, of 9 to 16 rows from 20 MB, of fewer from 40 MB; below, and where K is a multiple of
+    32, the mma.sync kernel.  Behind a norm kernel, in replayed graphs with other weights, in us, before / here: 17 MB with
+    K = 896 at 8 / 9 / 16 / 32 / 64 rows 6.6 / 8.8 / 9.0 / 11.9 / 14.7 against 9.0 / 9.0 / 9.2 / 9.4 / 10.1; 23 MB 8.7 / 13.1 / 13.7 /
+    16.0 / 19.7 against 11.2 / 11.2 / 11.3 / 11.2 / 12.4; 46 MB with K = 2,048 15.7 / 16.3 / 17.1 / 18.1 / 21.1 against 13.5 / 13.5 / 13.7 /
+    13.8 / 15.0; 55 MB 15.4 / 15.1 / 16.0 / 17.0 / 19.9 against 13.8 / 14.0 / 14.1 / 15.0 / 16.7; 100 MB 22.6 / 22.7 / 24.2 / 26.2 / 29.5
+    against 20.7 / 20.8 / 21.3 / 22.2 / 24.0; 272 MB 44.7 / 44.9 / 46.0 / 47.8 / 52.3 against 45.6 / 45.9 / 46.7 / 48.3 / 51.8; 566 MB 91.6 /
+    91.4 / 93.6 / 97.0 / 105.7 against 87.1 / 87.3 / 88.2 / 90.5 / 94.1."""
+    size = w.numel() * 2
+    if rows > ROW_KERNEL_MAX_ROWS or w.shape[1] % 32:
+        return True
+    return size >= (PAIR_MIN_BYTES_ROWS if rows > 8 else PAIR_MIN_BYTES)
 
 
 def _gate(swiglu, activation) -> int:
@@ -179,12 +200,24 @@ def gemm_tc(x, w, out, bias=None, epilogue=EPI_STORE):
 def decode_gemm_tc(x, w, out, bias=None, accumulate=False, swiglu=False, activation=elementwise.ACT_SILU):
     """bfloat16 x [M <= 64, K] times w [N, K]^T on the tcgen05 tensor cores
     with the operands swapped (csrc/decode_gemm_tc.cu): the weight streams once
-    through TMA, K is split over a thread-block cluster where tiles are few."""
+    through TMA, K is split over a thread-block cluster where tiles are few.  Gated products: `decode_pair_tc`."""
+    if swiglu:
+        return decode_pair_tc(x, w, out, bias, accumulate, activation)
     M, K = x.shape
     N = out.shape[1]
     check(core().tq_decode_gemm_tc(ptr(x), ptr(w), ptr(bias), ptr(out), dtype_code(out), M, N, K, x.stride(0),
                                    w.stride(0), out.stride(0), int(accumulate), _gate(swiglu, activation),
                                    ptr(tc_status_word(x.device)), stream()), "decode_gemm_tc")
+    return out
+
+
+def decode_pair_tc(x, w, out, bias=None, accumulate=False, activation=elementwise.ACT_SILU):
+    """out (=, +=) act(x · gate^T) * (x · up^T) for bfloat16 x [M <= 64, K] and w [2N, K] (gate rows, then up rows) on the tcgen05
+    tensor cores, the columns cut so that every SM reads the same share of w once (csrc/decode_pair_tc.cu)."""
+    M, K = x.shape
+    check(core().tq_decode_pair_tc(ptr(x), ptr(w), ptr(bias), ptr(out), dtype_code(out), M, out.shape[1], K, x.stride(0),
+                                   w.stride(0), out.stride(0), int(accumulate), int(activation),
+                                   ptr(tc_status_word(x.device)), stream()), "decode_pair_tc")
     return out
 
 
@@ -338,12 +371,15 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = N
             and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and out.dtype in (torch.float32, torch.bfloat16) and (not accumulate or out.dtype == torch.float32)):
         return row_gemm(x, w, out, bias, accumulate, swiglu, activation, w_settled)
-    # decoding: the TMA-fed tcgen05 kernel or the mma.sync kernel (_tc_takes says which, where both can)
-    if (USE_TCGEN05 and M <= SKINNY_MAX_ROWS and _tc_ok(x, w, out, swiglu)
+    # decoding: a TMA-fed tcgen05 kernel or the mma.sync kernel (_pair_takes and _tc_takes say which, where both can)
+    if (swiglu and USE_TCGEN05 and M <= SKINNY_MAX_ROWS and _tc_ok(x, w, out, swiglu)
+            and (not accumulate or out.dtype == torch.float32) and (not _skinny_ok(x, w) or _pair_takes(M, w))):
+        return decode_pair_tc(x, w, out, bias, accumulate, activation)
+    if (not swiglu and USE_TCGEN05 and M <= SKINNY_MAX_ROWS and _tc_ok(x, w, out, swiglu)
             and (not accumulate or out.dtype == torch.float32) and not (relu2 and out.dtype != torch.bfloat16)
             and (not _skinny_ok(x, w)
-                 or _tc_takes(M, w, bool(swiglu), pending is not None, out.dtype == torch.float32))):
-        return decode_gemm_tc(x, w, out, bias, accumulate, swiglu, activation)
+                 or _tc_takes(M, w, False, pending is not None, out.dtype == torch.float32))):
+        return decode_gemm_tc(x, w, out, bias, accumulate, False, activation)
     if _skinny_ok(x, w):
         return skinny_gemm(x, w, out, bias, accumulate, swiglu, activation)
     if _f32_ok(x, w, out):
