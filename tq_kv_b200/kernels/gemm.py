@@ -18,7 +18,8 @@
     the reference engine does for all its products
     (src/models/turbo_generic.rs:68-91 -> candle -> cuBLAS);
   * float32 operands and result (the float32 path): the FMA kernels of
-    csrc/gemm_f32.cu with the same epilogues, for up to 8 rows and for more;
+    csrc/gemm_f32.cu with the same epilogues, for up to 8 rows and for more; many rows (`_f32_tc_takes`) on tcgen05
+    with every number split exactly into three bfloat16 parts (csrc/gemm_f32_tc.cu);
   * everything else (mixed operands, rows that are not 16-byte aligned): the
     row kernel and the tiled FMA kernel of csrc/gemm.cu.  Never a
     reduced-precision mode.
@@ -314,6 +315,25 @@ def _f32_ok(x, w, out) -> bool:
             and (x.shape[0] == 1 or (x.stride(0) >= K and out.stride(0) >= out.shape[1])) and w.stride(0) >= K)
 
 
+def _f32_tc_takes(rows: int, columns: int, gated: bool) -> bool:
+    """Which float32 products run on csrc/gemm_f32_tc.cu (its error against 64 bits is no larger): of more than 128 rows all, of
+    more than 32 those with at least 8 tiles of 256 columns (128 of a gated product).  In us, the FMA tiles / there: 300 rows,
+    N = K = 896 18.8 / 15.6, N = 1,152 21.6 / 16.3; 100 rows, N = 896, K = 896 11.9 / 14.2 and K = 4,864 37 / 41, N = K = 2,048
+    30.7 / 22.2; 64 rows, N = 1,152 12.0 / 13.4, N = K = 2,048 29.9 / 20.6, N = 8,224 56 / 35, N = 151,936 404 / 282; 32 rows, N = 8,224
+    33.7 / 33.6, N = K = 2,048 17.6 / 19.6, N = 151,936 237 / 268."""
+    return USE_TCGEN05 and (rows > 128 or (rows > 32 and columns > 7 * (128 if gated else 256)))
+
+
+def gemm_f32_tc(x, w, out, bias=None, accumulate=False, swiglu=False, activation=elementwise.ACT_SILU, w_settled=False):
+    """float32 x [M, K] times w [N, K]^T on the tcgen05 tensor cores, three exact bfloat16 parts a number
+    (csrc/gemm_f32_tc.cu).  `w_settled`: see `linear`."""
+    M, K = x.shape
+    check(core().tq_gemm_f32_tc(ptr(x), ptr(w), ptr(bias), ptr(out), M, out.shape[1], K, x.stride(0), w.stride(0), out.stride(0),
+                                int(accumulate), _gate(swiglu, activation), int(w_settled), ptr(tc_status_word(x.device)),
+                                stream()), "gemm_f32_tc")
+    return out
+
+
 def gemm_f32(x, w, out, bias=None, accumulate=False, swiglu=False, activation=elementwise.ACT_SILU, w_settled=False):
     """float32 x [M, K] times w [N, K]^T on FMA units (csrc/gemm_f32.cu): up to 8 rows by the kernel that streams w
     once, more by tiles.  `w_settled`: see `linear`."""
@@ -383,6 +403,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = N
     if _skinny_ok(x, w):
         return skinny_gemm(x, w, out, bias, accumulate, swiglu, activation)
     if _f32_ok(x, w, out):
+        if _f32_tc_takes(M, N, bool(swiglu)):
+            return gemm_f32_tc(x, w, out, bias, accumulate, swiglu, activation, w_settled)
         return gemm_f32(x, w, out, bias, accumulate, swiglu, activation, w_settled)
     if M <= ROW_KERNEL_MAX_ROWS:
         return gemv_rows(x, w, out, bias, accumulate, swiglu, activation)
