@@ -10,38 +10,7 @@
 // block writes (unnormalised output, max, sum) for attention_merge_kernel.
 //
 // Formulas: src/models/turbo_generic.rs:1620-1631 (see attention.cu).
-#include "common.cuh"
-
-#define FD_WARPS 4
-#define FD_STAGES 3
-#define FD_PAGE 64           // tokens per cache page (checked by the launcher)
-
-__device__ __forceinline__ void fd_mma(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-    asm(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void fd_ldmatrix_x4(uint32_t* r, const void* smem) {
-    const uint32_t addr = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void fd_ldmatrix_x4_trans(uint32_t* r, const void* smem) {
-    const uint32_t addr = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void fd_cp_async16(void* smem, const void* gmem) {
-    const uint32_t addr = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(addr), "l"(gmem));
-}
-__device__ __forceinline__ void fd_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N> __device__ __forceinline__ void fd_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-__device__ __forceinline__ uint32_t fd_pack(float a, float b) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&v);
-}
+#include "flash_decode.cuh"
 
 // What becomes of a chunk's scores.  FD_SOFTMAX: the online softmax described above.  FD_SIGMOID: the weight of key
 // j for the token at position i and head h is sigmoid(score * scale + bias[h, min(i - j, n_dist - 1)]) (a float32

@@ -123,6 +123,47 @@ def attention(q: torch.Tensor, out: torch.Tensor, *, n_heads: int, n_kv_heads: i
     return out
 
 
+ROPE_DECODE_WIDTHS = (32, 64)     # head widths of the kernel that does a decode step's attention whole
+ROPE_DECODE_MAX_KEYS = 4096      # of the longest range: beyond, the separate kernels cut it into more than 8 splits
+
+
+def rope_decode_splits(n_tokens: int, n_heads: int, n_kv_heads: int, head_dim: int, max_keys: int, page_tokens: int,
+                       sm_count: int) -> int:
+    """Blocks a (token, key/value head) of `rope_decode` for a step of single tokens: as many as `plan_splits` gives, down to
+    a power of two up to 8; 0 where the separate kernels run (wider heads, pages outside its reach, more than
+    ROPE_DECODE_MAX_KEYS keys that they would cut into 9 or more; measured: csrc/rope_decode.cu)."""
+    if (head_dim not in ROPE_DECODE_WIDTHS or n_heads // n_kv_heads > 16 or page_tokens != 64 or n_kv_heads > 65535
+            or n_tokens > 65535):
+        return 0
+    n = plan_splits(n_tokens, n_kv_heads, max_keys, sm_count)
+    if n > 8 and max_keys > ROPE_DECODE_MAX_KEYS:
+        return 0
+    return 8 if n >= 8 else 4 if n >= 4 else 2 if n >= 2 else 1
+
+
+def rope_decode(qkv, bias, cos, sin, out, *, n_heads, n_kv_heads, head_dim, rotary_dim, k_pages, v_pages, block_table,
+                table_width, ring_pages, page_tokens, tok_pos, tok_seq, new_lens, window, n_splits, clear_input=False):
+    """One kernel for a decode step's rotary encoding, cache append and attention (csrc/rope_decode.cu): qkv float32
+    [T, (nh + 2 nkv) * hd], every row its sequence's only token of the step; out bfloat16 [T, nh * hd].  `n_splits`: see
+    `rope_decode_splits`.  With `clear_input` the kernel leaves zeros in qkv."""
+    T = qkv.shape[0]
+    width = (n_heads + 2 * n_kv_heads) * head_dim
+    if qkv.dtype != torch.float32 or qkv.shape[1] != width or out.dtype != torch.bfloat16 or tuple(out.shape) != (T, n_heads * head_dim):
+        raise KernelError(f"rope_decode: qkv float32 [T, {width}], out bfloat16 [T, {n_heads * head_dim}]")
+    if k_pages.dtype != torch.bfloat16 or v_pages.dtype != torch.bfloat16 or tuple(k_pages.shape[1:]) != (n_kv_heads, page_tokens, head_dim):
+        raise KernelError(f"rope_decode: bfloat16 cache pages [pages, {n_kv_heads}, {page_tokens}, {head_dim}]")
+    if cos.dtype != torch.float32 or sin.dtype != torch.float32 or cos.shape[1] != rotary_dim // 2:
+        raise KernelError("rope_decode: cos/sin must be float32 [positions, rotary_dim/2]")
+    if bias is not None and (bias.dtype != torch.float32 or bias.shape[0] != width):
+        raise KernelError("rope_decode: bias must be float32 of the qkv width")
+    need_contiguous(qkv=qkv, bias=bias, cos=cos, sin=sin, out=out, k_pages=k_pages, v_pages=v_pages, block_table=block_table)
+    check(core().tq_rope_decode(ptr(qkv), ptr(bias), ptr(cos), ptr(sin), ptr(k_pages), ptr(v_pages), ptr(block_table), table_width,
+                                ring_pages, page_tokens, ptr(tok_pos), ptr(tok_seq), ptr(new_lens), int(window or 0),
+                                1.0 / math.sqrt(head_dim), ptr(out), T, n_heads, n_kv_heads, head_dim, rotary_dim, n_splits,
+                                int(clear_input), stream()), "rope_decode")
+    return out
+
+
 def check_row_widths(n_heads: int, n_kv_heads: int, key_dim: int, value_dim: int) -> None:
     """Raises for head sizes the general attention kernel with options does not take."""
     for name, d in (("key", key_dim), ("value", value_dim)):

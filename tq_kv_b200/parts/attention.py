@@ -125,6 +125,25 @@ class GQAttention(Mixer):
         else:
             qkv = kernels.linear(x, self.w_qkv, out_dtype=torch.float32, w_settled=True)
         kernels.mark("qkv")
+        # A decode step of single tokens: rotary encoding, cache append and attention are one kernel where it takes the shape.
+        tables = getattr(self.position, "decode_tables", lambda: None)()
+        if owns and not packed and act == torch.bfloat16 and tables is not None and b.single_tokens:
+            max_keys = b.max_new_len if self.window is None else min(b.max_new_len, self.window)
+            splits = kernels.rope_decode_splits(T, self.n_heads, self.n_kv_heads, self.head_dim, max_keys, kv.page_tokens,
+                                                ctx.runtime.sm_count)
+            if splits:
+                out = torch.empty((T, self.q_width), dtype=act, device=dev)
+                kernels.rope_decode(qkv, self.b_qkv, *tables[:2], out, n_heads=self.n_heads, n_kv_heads=self.n_kv_heads,
+                                    head_dim=self.head_dim, rotary_dim=tables[2], k_pages=kv.k_pages, v_pages=kv.v_pages,
+                                    block_table=kv.block_table, table_width=kv.table_width, ring_pages=kv.ring_pages,
+                                    page_tokens=kv.page_tokens, tok_pos=b.tok_pos, tok_seq=b.tok_seq, new_lens=b.new_lens,
+                                    window=self.window, n_splits=splits, clear_input=kept_zero)
+                if kept_zero:
+                    self._qkv_zero[1][0] = False
+                kernels.mark("attention")
+                kernels.linear(out, self.w_o, bias=self.b_o, out=residual, accumulate=True, w_settled=True)
+                kernels.mark("o")
+                return
         q = torch.empty((T, self.q_width), dtype=act, device=dev)
         k = torch.empty((T, self.kv_width), dtype=act, device=dev) if packed else None
         v = torch.empty((T, self.kv_width), dtype=act, device=dev) if packed else None

@@ -50,6 +50,12 @@ class RotaryHalved(PositionEncoding):
 
     clears_input = True          # encode_and_store(..., clear_input=True) leaves zeros in qkv
 
+    def decode_tables(self):
+        """(cos, sin, rotary_dim) for a mixer that runs a decode step's encoding, cache append and attention as one kernel;
+        None where a subclass encodes in its own way."""
+        own = type(self).encode_and_store is RotaryHalved.encode_and_store
+        return (self.cos, self.sin, self.rotary_dim) if own else None
+
     def encode_and_store(self, qkv, bias, ctx: StepContext, *, n_heads, n_kv_heads, head_dim, q_out, k_out, v_out,
                          clear_input=False):
         b = ctx.batch
