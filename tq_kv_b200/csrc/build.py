@@ -26,7 +26,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 
 GROUPS: dict[str, list[str]] = {
     # everything a model needs in either precision
-    "core": ["elementwise.cu", "attention.cu", "flash_decode.cu", "rope_decode.cu", "flash_prefill.cu", "flash_prefill_tc.cu", "gemm.cu", "gemm_f32.cu", "gemm_f32_tc.cu", "skinny_gemm.cu", "row_gemm.cu",
+    "core": ["elementwise.cu", "attention.cu", "flash_decode.cu", "rope_decode.cu", "flash_prefill.cu", "prompt_attention_f32.cu", "flash_prefill_tc.cu", "gemm.cu", "gemm_f32.cu", "gemm_f32_tc.cu", "skinny_gemm.cu", "row_gemm.cu",
              "gemm_tc.cu", "decode_gemm_tc.cu", "decode_pair_tc.cu", "sampling.cu", "random_fill.cu", "linear_scan.cu", "block_scan.cu", "sigmoid_attention.cu",
              "short_conv.cu", "latent_attention.cu", "head_encode.cu", "stream_mix.cu", "routed_experts.cu", "mlstm.cu",
              "gru_scan.cu", "low_rank.cu", "channel_scan.cu"],

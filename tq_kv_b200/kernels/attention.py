@@ -115,6 +115,15 @@ def attention(q: torch.Tensor, out: torch.Tensor, *, n_heads: int, n_kv_heads: i
                 check(core().tq_attention_merge(ptr(part_acc), ptr(part_ml), ptr(out), dtype_code(out), T, n_heads,
                                                 head_dim, n_splits, 0, stream()), "attention_merge")
             return out
+    if q.dtype == torch.float32 and use_flash and T > n_seqs and n_splits == 1:
+        # float32 prompts: 64 rows a block over the same keys (with the keys split the general kernel has more blocks)
+        st = core().tq_prompt_attention_f32(
+            ptr(q), ptr(k_packed), ptr(v_packed), ptr(k_pages), ptr(v_pages), ptr(block_table), table_width, ring_pages,
+            page_tokens, ptr(tok_pos), ptr(tok_seq), ptr(cu_seqlens), ptr(start_pos), int(window or 0), float(scale), ptr(out), T,
+            n_heads, n_kv_heads, head_dim, stream())
+        if st != NOT_SUPPORTED:
+            check(st, "prompt_attention_f32")
+            return out
     check(core().tq_attention(
         ptr(q), dtype_code(q), ptr(k_packed), ptr(v_packed), ptr(k_pages), ptr(v_pages), ptr(block_table),
         table_width, ring_pages, page_tokens, ptr(tok_pos), ptr(tok_seq), ptr(cu_seqlens), ptr(start_pos),
