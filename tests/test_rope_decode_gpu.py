@@ -23,8 +23,8 @@ def _setup(lens, nh, nkv, hd, rot, ring=0, seed=0):
                 pos=i32([n - 1 for n in lens]), seq=i32(list(range(T))), new=i32(lens), cu=i32(list(range(T + 1))))
 
 
-def _wanted(s, nh, nkv, hd, rot, window, ring, bias):
-    """float64 from the step's row and the cache; the new key and value rounded as they are cached."""
+def _wanted(s, nh, nkv, hd, rot, window, ring, bias, dtype=torch.bfloat16):
+    """float64 from the step's row and the cache; q and the new key and value rounded as they are cached."""
     outs = []
     for t, pos in enumerate(s["pos"].tolist()):
         x = (s["qkv"][t] + (s["bias"] if bias else 0)).double().reshape(nh + 2 * nkv, hd)
@@ -32,7 +32,7 @@ def _wanted(s, nh, nkv, hd, rot, window, ring, bias):
         h = x[:nh + nkv].clone()
         a, b = x[:nh + nkv, :rot // 2], x[:nh + nkv, rot // 2:rot]
         h[:, :rot // 2], h[:, rot // 2:rot] = a * c - b * n, a * n + b * c
-        q, k_new, v_new = h[:nh].bfloat16().double(), h[nh:].bfloat16(), x[nh + nkv:].bfloat16()
+        q, k_new, v_new = h[:nh].to(dtype).double(), h[nh:].to(dtype), x[nh + nkv:].to(dtype)
         lo = max(0, pos - window + 1) if window else 0
         js = torch.arange(lo, pos, device=DEV)
         lp = js // 64 % ring if ring else js // 64
@@ -70,6 +70,30 @@ def test_beside_float64_and_the_separate_kernels(nh, nkv, hd, rot, lens, window,
     assert bool((row == 0).all()) if splits == 4 else torch.equal(row, s["qkv"])
     # weights are rounded to bfloat16 before they meet the values (2^-9 of a sum of values around one), and so is the result
     assert float((out.double() - want).abs().max()) < 2.0 ** -7 * float(want.abs().max()) + 2.0 ** -8
+
+
+@pytest.mark.parametrize("nh,nkv,hd,rot", [(14, 2, 64, 64), (28, 2, 64, 62), (4, 4, 32, 16), (16, 1, 32, 32)])
+@pytest.mark.parametrize("lens,window,ring", [([1], None, 0), ([33, 2, 32, 64], None, 0), ([65, 300, 1000], None, 0), ([700, 130], 100, 3)])
+@pytest.mark.parametrize("splits", [1, 2, 8])
+def test_float32_beside_float64_and_the_separate_kernels(nh, nkv, hd, rot, lens, window, ring, splits):
+    from tq_kv_b200 import kernels
+    s = _setup(lens, nh, nkv, hd, rot, ring, seed=sum(lens) + hd)
+    s["k"], s["v"] = s["k"].float(), s["v"].float()
+    T, bias = len(lens), s["bias"] if splits != 2 else None
+    common = dict(n_heads=nh, n_kv_heads=nkv, head_dim=hd)
+    cache = dict(block_table=s["table"], table_width=s["width"], ring_pages=ring)
+    want = _wanted(s, nh, nkv, hd, rot, window, ring, bias is not None, torch.float32)
+    k0, v0 = s["k"].clone(), s["v"].clone()
+    q, apart, out = (torch.full((T, nh * hd), 7.0, device=DEV) for _ in range(3))
+    kernels.qkv_rope_cache(s["qkv"], bias, s["cos"], s["sin"], s["pos"], s["seq"], s["new"], q, rotary_dim=rot, k_pages=k0, v_pages=v0,
+                           **cache, **common)
+    kernels.attention(q, apart, tok_pos=s["pos"], tok_seq=s["seq"], cu_seqlens=s["cu"], start_pos=s["pos"], window=window, k_pages=k0,
+                      v_pages=v0, **cache, **common)
+    kernels.rope_decode(s["qkv"], bias, s["cos"], s["sin"], out, rotary_dim=rot, k_pages=s["k"], v_pages=s["v"], page_tokens=64,
+                        tok_pos=s["pos"], tok_seq=s["seq"], new_lens=s["new"], window=window, n_splits=splits, **cache, **common)
+    assert torch.equal(s["v"], v0) and float((s["k"].double() - k0.double()).abs().max()) <= 2.0 ** -22 * float(k0.abs().max())
+    err, err_apart = (float((x.double() - want).norm() / want.norm()) for x in (out, apart))
+    assert err <= max(1.5 * err_apart, 4e-7), (err, err_apart)       # float32 sums of the same numbers in another order
 
 
 def test_a_row_past_its_sequences_new_length_is_not_cached():

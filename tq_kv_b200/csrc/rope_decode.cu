@@ -369,3 +369,247 @@ TQ_API int tq_rope_decode(float* qkv, const float* bias, const float* cos_tab, c
         default: return (int)cudaErrorNotSupported;
     }
 }
+
+// ---- float32 ------------------------------------------------------------------------------------------------------
+// The same in float32 throughout (multiply-adds; weights of the softmax included): pieces of 32 keys and values in shared
+// memory, two stages, fetched by the whole block; a warp serves the q heads w, w + 8 of the group: a lane a key for the scores,
+// a lane HD / 32 dims for the values.  The separate kernels (rotary, general attention, merge) took 3.2 + 13.9 + 2.5 us a layer for
+// two sequences of 160 keys, 14 heads on 2 of 64; 6.4 here.
+#define RF_KEYS 32
+#define RF_THREADS 256
+
+struct RopeDecodeF32Args {
+    const float *qkv, *bias, *cos_tab, *sin_tab;
+    float *k_pages, *v_pages;
+    const int *block_table, *tok_pos, *tok_seq, *new_lens;
+    float* out;
+    int table_width, ring_pages, window, nh, nkv, rot;
+    float scale;
+};
+
+template <int HD, int HPW>
+__global__ void __launch_bounds__(RF_THREADS) rope_decode_f32_kernel(const RopeDecodeF32Args a) {
+    namespace cg = cooperative_groups;
+    constexpr int LD = HD + 4, TILE = RF_KEYS * LD, DV = HD / 32, RS = HD + 2;
+    extern __shared__ __align__(16) float fsh[];
+    float *stages = fsh, *qs = stages + 4 * TILE, *part = qs + 8 * HPW * LD;       // stages: [2][keys, values]
+    cg::cluster_group cluster = cg::this_cluster();
+    const int n_ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int t = blockIdx.z, g = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n_rep = a.nh / a.nkv;
+    const int pos = a.tok_pos[t], b = a.tok_seq[t];
+    const int lo_all = (a.window > 0 && pos - a.window + 1 > 0) ? pos - a.window + 1 : 0;
+    const int n_old = pos - lo_all, split_len = (n_old + n_ranks - 1) / n_ranks;
+    const int lo = min(n_old, rank * split_len), hi = min(n_old, lo + split_len);
+    const int n_tiles = (hi - lo + RF_KEYS - 1) / RF_KEYS;
+    const int* table = a.block_table + (size_t)b * a.table_width;
+    auto cache_row = [&](int j) {
+        int lp = j / FD_PAGE;
+        if (a.ring_pages > 0) lp %= a.ring_pages;
+        return (((unsigned long long)table[lp] * a.nkv + g) * FD_PAGE + (j % FD_PAGE)) * HD;
+    };
+    auto issue = [&](int i) {
+        if (i < n_tiles) {
+            float* dst = stages + (i & 1) * 2 * TILE;
+            for (int e = threadIdx.x; e < RF_KEYS * (HD / 4); e += RF_THREADS) {
+                const int key = e / (HD / 4), c = e % (HD / 4) * 4;
+                const unsigned long long row = cache_row(lo_all + min(lo + i * RF_KEYS + key, hi - 1)) + c;
+                fd_cp_async16(dst + key * LD + c, a.k_pages + row);
+                fd_cp_async16(dst + TILE + key * LD + c, a.v_pages + row);
+            }
+        }
+        fd_commit();
+    };
+    issue(0);
+    const int half = a.rot >> 1;
+    const float *cs = a.cos_tab + (size_t)pos * half, *sn = a.sin_tab + (size_t)pos * half;
+    const float* row = a.qkv + (size_t)t * (a.nh + 2 * a.nkv) * HD;
+    const bool keep = rank == 0 && pos < a.new_lens[b];
+    const unsigned long long new_row = keep ? cache_row(pos) : 0;
+    float* hold = part + 16 * RS;                          // rank 0: the new key, the new value
+    // What a thread turns: pairs e = thread, thread + threads, ... of (head, pair), the q heads of the group and (rank 0) the key,
+    // then the value's entries, PER at a time: what does not depend on the kernel in front is loaded before it ends, then all of
+    // the row's entries at once (one after the other they took longer than the attention).
+    constexpr int PER = 4;
+    const int turned = (n_rep + (rank == 0 ? 1 : 0)) * (HD / 2), work = turned + (rank == 0 ? HD / 2 : 0);
+    const float* bias = a.bias;
+    bool waited = false;
+    for (int e0 = threadIdx.x; e0 < work || !waited; e0 += PER * RF_THREADS) {
+        int at0[PER], at1[PER];                            // the two entries of the row
+        float c[PER], s[PER], b0[PER], b1[PER], u0[PER], u1[PER];
+#pragma unroll
+        for (int p = 0; p < PER; ++p) {
+            const int e = e0 + p * RF_THREADS, r = e / (HD / 2), i = e - r * (HD / 2);
+            const int head = r < n_rep ? g * n_rep + r : e < turned ? a.nh + g : a.nh + a.nkv + g;
+            const bool turns = e < turned && i < half;
+            const int d0 = e >= turned ? 2 * i : turns ? i : a.rot + 2 * (i - half);
+            at0[p] = e < work ? head * HD + d0 : -1;
+            at1[p] = at0[p] + (turns ? half : 1);
+            c[p] = e < work && turns ? cs[i] : 1.f;
+            s[p] = e < work && turns ? sn[i] : 0.f;
+            b0[p] = e < work && bias ? bias[at0[p]] : 0.f;
+            b1[p] = e < work && bias ? bias[at1[p]] : 0.f;
+        }
+        if (!waited) pdl_wait();
+        waited = true;
+#pragma unroll
+        for (int p = 0; p < PER; ++p) {
+            u0[p] = at0[p] >= 0 ? row[at0[p]] : 0.f;
+            u1[p] = at0[p] >= 0 ? row[at1[p]] : 0.f;
+        }
+#pragma unroll
+        for (int p = 0; p < PER; ++p) {
+            if (at0[p] < 0) continue;
+            const int e = e0 + p * RF_THREADS, r = e / (HD / 2);
+            const int d0 = at0[p] % HD, d1 = at1[p] % HD;
+            const bool turns = e < turned && e - r * (HD / 2) < half;
+            const float x0 = u0[p] + b0[p], x1 = u1[p] + b1[p];
+            const float y0 = (turns ? fmaf(x0, c[p], -__fmul_rn(x1, s[p])) : x0), y1 = (turns ? fmaf(x0, s[p], __fmul_rn(x1, c[p])) : x1);
+            float* dst = r < n_rep ? qs + r * LD : e < turned ? hold : hold + HD;
+            dst[d0] = y0;
+            dst[d1] = y1;
+            if (keep && r >= n_rep) {
+                float* page = (e < turned ? a.k_pages : a.v_pages) + new_row;
+                page[d0] = y0;
+                page[d1] = y1;
+            }
+        }
+    }
+    float m[HPW], l[HPW], acc[HPW][DV];
+#pragma unroll
+    for (int h = 0; h < HPW; ++h) {
+        m[h] = -INFINITY;
+        l[h] = 0.f;
+#pragma unroll
+        for (int c = 0; c < DV; ++c) acc[h][c] = 0.f;
+    }
+    // keys and values at kt and vt (rows LD apart), the first `live` of them count (at least one)
+    auto attend = [&](const float* kt, const float* vt, int live) {
+#pragma unroll
+        for (int h = 0; h < HPW; ++h) {
+            const int r = warp + 8 * h;
+            if (r >= n_rep) continue;
+            float s = -INFINITY;
+            if (lane < live) {
+                float dot = 0.f;
+#pragma unroll 8
+                for (int d = 0; d < HD; d += 4) {
+                    const float4 x = *reinterpret_cast<const float4*>(qs + r * LD + d);
+                    const float4 k = *reinterpret_cast<const float4*>(kt + lane * LD + d);
+                    dot = fmaf(x.x, k.x, dot); dot = fmaf(x.y, k.y, dot);
+                    dot = fmaf(x.z, k.z, dot); dot = fmaf(x.w, k.w, dot);
+                }
+                s = dot * a.scale;
+            }
+            const float m_new = fmaxf(m[h], warp_max(s));
+            const float p = lane < live ? expf(s - m_new) : 0.f, corr = expf(m[h] - m_new);
+            l[h] = l[h] * corr + warp_sum(p);
+            m[h] = m_new;
+#pragma unroll
+            for (int c = 0; c < DV; ++c) acc[h][c] *= corr;
+#pragma unroll 4
+            for (int j = 0; j < live; ++j) {
+                const float pj = __shfl_sync(0xffffffffu, p, j);
+#pragma unroll
+                for (int c = 0; c < DV; ++c) acc[h][c] = fmaf(pj, vt[j * LD + lane + 32 * c], acc[h][c]);
+            }
+        }
+    };
+    for (int i = 0; i < n_tiles; ++i) {
+        issue(i + 1);
+        fd_wait<1>();
+        __syncthreads();                                   // the piece (and at first q) is there for all
+        const float* kt = stages + (i & 1) * 2 * TILE;
+        attend(kt, kt + TILE, min(RF_KEYS, hi - lo - i * RF_KEYS));
+        __syncthreads();                                   // the stage may be filled again
+    }
+    fd_wait<0>();
+    pdl_launch();
+    __syncthreads();
+    if (rank == 0) attend(hold, hold + HD, 1);
+#pragma unroll
+    for (int h = 0; h < HPW; ++h) {
+        const int r = warp + 8 * h;
+        if (r >= n_rep) continue;
+#pragma unroll
+        for (int c = 0; c < DV; ++c) part[r * RS + lane + 32 * c] = acc[h][c];
+        if (lane == 0) { part[r * RS + HD] = m[h]; part[r * RS + HD + 1] = l[h]; }
+    }
+    if (n_ranks > 1) cluster.sync();
+    else __syncthreads();
+    float* out = a.out + ((size_t)t * a.nh + (size_t)g * n_rep) * HD;
+    for (int e = rank * RF_THREADS + threadIdx.x; e < n_rep * HD; e += n_ranks * RF_THREADS) {
+        const int r = e / HD, d = e - r * HD;
+        float pm[RD_MAX_SPLITS], pl[RD_MAX_SPLITS], pv[RD_MAX_SPLITS], top = -INFINITY, sum = 0.f, v = 0.f;
+#pragma unroll
+        for (int p = 0; p < RD_MAX_SPLITS; ++p) {
+            const float* x = p < n_ranks ? (n_ranks > 1 ? cluster.map_shared_rank(part, p) : part) + r * RS : nullptr;
+            pm[p] = x ? x[HD] : -INFINITY;
+            pl[p] = x ? x[HD + 1] : 0.f;
+            pv[p] = x ? x[d] : 0.f;
+            top = fmaxf(top, pm[p]);
+        }
+#pragma unroll
+        for (int p = 0; p < RD_MAX_SPLITS; ++p)
+            if (pm[p] > -INFINITY) {
+                const float f = expf(pm[p] - top);
+                sum += pl[p] * f;
+                v += pv[p] * f;
+            }
+        out[e] = v / sum;
+    }
+    if (n_ranks > 1) cluster.sync();                       // nobody leaves while its results are being read
+}
+
+template <int HD, int HPW>
+static int launch_rope_decode_f32(const RopeDecodeF32Args& a, int n_tokens, int n_splits, cudaStream_t stream) {
+    constexpr size_t smem = (4 * RF_KEYS * (HD + 4) + 8 * HPW * (HD + 4) + 16 * (HD + 2) + 2 * HD) * sizeof(float);
+    static bool configured[64] = {false};                  // per device: the attribute belongs to its copy of the kernel
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
+    if (!configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(rope_decode_f32_kernel<HD, HPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        configured[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(n_splits, a.nkv, n_tokens);
+    cfg.blockDim = dim3(RF_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = tq_pdl_enabled(TQ_PDL_FLASH_DECODE) ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = n_splits;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, rope_decode_f32_kernel<HD, HPW>, a);
+    if (e != cudaSuccess) return (int)e;
+    return tq_launch_status();
+}
+
+// As tq_rope_decode with float32 pages and result; the rows of qkv stay as they are.
+TQ_API int tq_rope_decode_f32(const float* qkv, const float* bias, const float* cos_tab, const float* sin_tab, float* k_pages,
+                              float* v_pages, const int* block_table, int table_width, int ring_pages, int page_tokens,
+                              const int* tok_pos, const int* tok_seq, const int* new_lens, int window, float scale, float* out,
+                              int n_tokens, int nh, int nkv, int hd, int rot, int n_splits, cudaStream_t stream) {
+    if (n_tokens <= 0) return 0;
+    if (nkv <= 0 || nh % nkv || nh / nkv > 16 || page_tokens != FD_PAGE || nkv > 65535 || n_tokens > 65535 || rot < 2 || rot % 2 ||
+        rot > hd || ((reinterpret_cast<uintptr_t>(k_pages) | reinterpret_cast<uintptr_t>(v_pages)) & 15))
+        return (int)cudaErrorNotSupported;
+    if (n_splits != 1 && n_splits != 2 && n_splits != 4 && n_splits != 8) return (int)cudaErrorInvalidValue;
+    if (!k_pages || !v_pages || !block_table) return (int)cudaErrorInvalidValue;
+    const RopeDecodeF32Args a{qkv, bias, cos_tab, sin_tab, k_pages, v_pages, block_table, tok_pos, tok_seq, new_lens, out,
+                              table_width, ring_pages, window, nh, nkv, rot, scale};
+#define TQ_RF(H) case H: return nh / nkv <= 8 ? launch_rope_decode_f32<H, 1>(a, n_tokens, n_splits, stream) : launch_rope_decode_f32<H, 2>(a, n_tokens, n_splits, stream)
+    switch (hd) {
+        TQ_RF(32);
+        TQ_RF(64);
+        default: return (int)cudaErrorNotSupported;
+    }
+#undef TQ_RF
+}

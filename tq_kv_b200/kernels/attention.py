@@ -153,23 +153,28 @@ def rope_decode_splits(n_tokens: int, n_heads: int, n_kv_heads: int, head_dim: i
 def rope_decode(qkv, bias, cos, sin, out, *, n_heads, n_kv_heads, head_dim, rotary_dim, k_pages, v_pages, block_table,
                 table_width, ring_pages, page_tokens, tok_pos, tok_seq, new_lens, window, n_splits, clear_input=False):
     """One kernel for a decode step's rotary encoding, cache append and attention (csrc/rope_decode.cu): qkv float32
-    [T, (nh + 2 nkv) * hd], every row its sequence's only token of the step; out bfloat16 [T, nh * hd].  `n_splits`: see
-    `rope_decode_splits`.  With `clear_input` the kernel leaves zeros in qkv."""
+    [T, (nh + 2 nkv) * hd], every row its sequence's only token of the step; out [T, nh * hd] and the pages bfloat16, or
+    float32 (then everything is).  `n_splits`: see `rope_decode_splits`.  With `clear_input` (bfloat16) the kernel leaves zeros
+    in qkv."""
     T = qkv.shape[0]
     width = (n_heads + 2 * n_kv_heads) * head_dim
-    if qkv.dtype != torch.float32 or qkv.shape[1] != width or out.dtype != torch.bfloat16 or tuple(out.shape) != (T, n_heads * head_dim):
-        raise KernelError(f"rope_decode: qkv float32 [T, {width}], out bfloat16 [T, {n_heads * head_dim}]")
-    if k_pages.dtype != torch.bfloat16 or v_pages.dtype != torch.bfloat16 or tuple(k_pages.shape[1:]) != (n_kv_heads, page_tokens, head_dim):
-        raise KernelError(f"rope_decode: bfloat16 cache pages [pages, {n_kv_heads}, {page_tokens}, {head_dim}]")
+    if qkv.dtype != torch.float32 or qkv.shape[1] != width or out.dtype not in (torch.bfloat16, torch.float32) \
+            or tuple(out.shape) != (T, n_heads * head_dim) or (clear_input and out.dtype == torch.float32):
+        raise KernelError(f"rope_decode: qkv float32 [T, {width}], out bfloat16 or float32 [T, {n_heads * head_dim}]")
+    if k_pages.dtype != out.dtype or v_pages.dtype != out.dtype or tuple(k_pages.shape[1:]) != (n_kv_heads, page_tokens, head_dim):
+        raise KernelError(f"rope_decode: cache pages of out's dtype [pages, {n_kv_heads}, {page_tokens}, {head_dim}]")
     if cos.dtype != torch.float32 or sin.dtype != torch.float32 or cos.shape[1] != rotary_dim // 2:
         raise KernelError("rope_decode: cos/sin must be float32 [positions, rotary_dim/2]")
     if bias is not None and (bias.dtype != torch.float32 or bias.shape[0] != width):
         raise KernelError("rope_decode: bias must be float32 of the qkv width")
     need_contiguous(qkv=qkv, bias=bias, cos=cos, sin=sin, out=out, k_pages=k_pages, v_pages=v_pages, block_table=block_table)
-    check(core().tq_rope_decode(ptr(qkv), ptr(bias), ptr(cos), ptr(sin), ptr(k_pages), ptr(v_pages), ptr(block_table), table_width,
-                                ring_pages, page_tokens, ptr(tok_pos), ptr(tok_seq), ptr(new_lens), int(window or 0),
-                                1.0 / math.sqrt(head_dim), ptr(out), T, n_heads, n_kv_heads, head_dim, rotary_dim, n_splits,
-                                int(clear_input), stream()), "rope_decode")
+    args = (ptr(qkv), ptr(bias), ptr(cos), ptr(sin), ptr(k_pages), ptr(v_pages), ptr(block_table), table_width, ring_pages,
+            page_tokens, ptr(tok_pos), ptr(tok_seq), ptr(new_lens), int(window or 0), 1.0 / math.sqrt(head_dim), ptr(out), T,
+            n_heads, n_kv_heads, head_dim, rotary_dim, n_splits)
+    if out.dtype == torch.float32:
+        check(core().tq_rope_decode_f32(*args, stream()), "rope_decode_f32")
+    else:
+        check(core().tq_rope_decode(*args, int(clear_input), stream()), "rope_decode")
     return out
 
 

@@ -127,7 +127,7 @@ class GQAttention(Mixer):
         kernels.mark("qkv")
         # A decode step of single tokens: rotary encoding, cache append and attention are one kernel where it takes the shape.
         tables = getattr(self.position, "decode_tables", lambda: None)()
-        if owns and not packed and act == torch.bfloat16 and tables is not None and b.single_tokens:
+        if owns and not packed and tables is not None and b.single_tokens:
             max_keys = b.max_new_len if self.window is None else min(b.max_new_len, self.window)
             splits = kernels.rope_decode_splits(T, self.n_heads, self.n_kv_heads, self.head_dim, max_keys, kv.page_tokens,
                                                 ctx.runtime.sm_count)
