@@ -126,6 +126,21 @@ decode_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const int k_lo = min(k_total, rank * k_per), k_hi = min(k_total, k_lo + k_per);
     const int k_iters = k_hi - k_lo;
 
+    auto load_w = [&](int i) {
+        const int s = i % DG_STAGES;
+        const uint32_t fb = dg_smem(&full[s]);
+        const uint32_t w_dst = dg_smem(tiles + s * STAGE_BYTES);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
+                     ::"r"(fb), "r"((uint32_t)(NORM ? DG_W_BYTES : STAGE_BYTES)) : "memory");
+        const int kc = (k_lo + i) * DG_BK;
+        if (SWIGLU) {
+            dg_tma(w_dst, &map_w, kc, n0, fb);                          // 64 gate rows
+            dg_tma(w_dst + DG_W_BYTES / 2, &map_w, kc, N + n0, fb);     // the 64 up rows of the same outputs
+        } else {
+            dg_tma(w_dst, &map_w, kc, n0, fb);
+        }
+    };
+    const int ahead = k_iters < DG_STAGES ? k_iters : DG_STAGES;         // the stages are empty at the start
     if (threadIdx.x == 0) {
         for (int s = 0; s < DG_STAGES; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(dg_smem(&full[s])), "r"(NORM ? 2u : 1u));
@@ -135,6 +150,11 @@ decode_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         *failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        // The weights do not depend on the kernel in front (see below): the first stages' are asked for while the block still
+        // sets itself up (after the tensor memory was there and all threads had met, they came about 1 us later: decode
+        // steps of the 7B shape with 1 / 8 / 64 sequences 2,655 -> 2,580, 2,925 -> 2,814, 3,403 -> 3,310 us, 0.5B 543 -> 532,
+        // zodosun-2k with 32 639 -> 621).
+        for (int i = 0; i < ahead; ++i) load_w(i);
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
@@ -147,30 +167,14 @@ decode_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const uint32_t tmem_base = *tmem_slot;
 
     // Programmatic dependent launch (common.cuh): the weights do not depend on the kernel before, so the first
-    // stages' W tiles are requested before waiting for it; X, bias and Y are touched only after pdl_wait().
+    // stages' W tiles were requested before waiting for it; X, bias and Y are touched only after pdl_wait().
     if (!(warp == 0 && lane == 0)) { pdl_wait(); pdl_launch(); }
     if (warp == 0 && lane == 0) {
         // ---- producer ----
-        auto load_w = [&](int i) {
-            const int s = i % DG_STAGES;
-            const uint32_t fb = dg_smem(&full[s]);
-            const uint32_t w_dst = dg_smem(tiles + s * STAGE_BYTES);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
-                         ::"r"(fb), "r"((uint32_t)(NORM ? DG_W_BYTES : STAGE_BYTES)) : "memory");
-            const int kc = (k_lo + i) * DG_BK;
-            if (SWIGLU) {
-                dg_tma(w_dst, &map_w, kc, n0, fb);                          // 64 gate rows
-                dg_tma(w_dst + DG_W_BYTES / 2, &map_w, kc, N + n0, fb);     // the 64 up rows of the same outputs
-            } else {
-                dg_tma(w_dst, &map_w, kc, n0, fb);
-            }
-        };
         auto load_x = [&](int i) {
             const int s = i % DG_STAGES;
             dg_tma(dg_smem(tiles + s * STAGE_BYTES) + DG_W_BYTES, &map_x, (k_lo + i) * DG_BK, 0, dg_smem(&full[s]));
         };
-        const int ahead = k_iters < DG_STAGES ? k_iters : DG_STAGES;     // the stages are empty at the start
-        for (int i = 0; i < ahead; ++i) load_w(i);
         pdl_wait();
         pdl_launch();
         if (!NORM)
