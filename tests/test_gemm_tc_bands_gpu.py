@@ -30,3 +30,10 @@ def test_bands(M, N, K):
     # a bfloat16 result: half a unit in its eighth bit, and the sums' error times the other factor
     assert bool(((out - want).abs() <= want.abs() * 2.0 ** -8 + tol * (1 + y.abs().max())).all())
     kernels.check_tc_status()
+
+
+@pytest.mark.parametrize("M", [257, 300, 385])
+@pytest.mark.parametrize("N,K", [(10304, 136), (3584, 1032)])
+def test_rows_of_few_tiles(M, N, K):
+    """Rows of two 256-row tiles on pairs of SMs and of three or four 128-row tiles on single ones: both forms, by size."""
+    test_bands(M, N, K)

@@ -28,8 +28,8 @@
 // reduce-add, so for those tiles the order of the float additions is not
 // fixed.
 //
-// From 129 rows on the same product runs on pairs of SMs (gemm_tc_pair_kernel
-// below): tcgen05.mma with cta_group::2 on 256 x 256 tiles, each block of a
+// From 129 rows on the same product mostly runs on pairs of SMs (gemm_tc_pair_kernel
+// below, tc_pairs): tcgen05.mma with cta_group::2 on 256 x 256 tiles, each block of a
 // 2-block cluster holding half of A's rows and half of the B tile, which cuts
 // what an SM loads per step from 48 to 32 KB (measured: 5 % off the prefill).
 #include <cuda.h>
@@ -713,7 +713,7 @@ static int launch_tc_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CU
                          ma, mb, mc, bias, M, N, K, b_rows_second, n_whole, parts, status);
 }
 
-// 0: pairs of SMs for products of more than 128 rows, single SMs otherwise; 1: single SMs always; 2: pairs always.
+// 0: pairs of SMs or single SMs as tc_pairs says; 1: single SMs always; 2: pairs always.
 // Starts from the environment variable TQ_GEMM_TC_MODE (a tuning aid), else 0.
 static int g_tc_mode = -1;
 TQ_API void tq_gemm_tc_mode(int mode) { g_tc_mode = mode; }
@@ -724,6 +724,26 @@ static int tc_mode() {
         if (g_tc_mode < 0 || g_tc_mode > 2) g_tc_mode = 0;
     }
     return g_tc_mode;
+}
+
+// Rounds of the SMs that a product takes: tiles over slots, the last round whole or (cut: float32 sums) in shares of K.
+static double tc_rounds(int n_tiles, int slots, int K, bool cut) {
+    double last = n_tiles % slots ? 1.0 : 0.0;
+    if (last > 0 && cut) tc_last_round_parts(n_tiles, slots, K, &last);
+    return n_tiles / slots + last;
+}
+
+// Whether a product runs on pairs of SMs.  A round on 256-row tiles of pairs takes as many SMs as one on 128-row tiles of single
+// SMs but is up to 20 % shorter (300 rows of a 2 x 18,944 x 3,584 product: four rounds 94 us, three 87); the last rows of a product,
+// though, fill a 256-row tile less well: 300 rows are 512 in one form and 384 in the other.  So single SMs run a product that
+// takes pairs more than 1.2 times its rounds (us on pairs / single SMs, 300 rows: 10,304 x 2,048 26.1 / 18.1, 2 x 5,632 x 2,048 26.2 /
+// 17.9, 3,584 x 3,584 summed into a residual 17.4 / 13.5, 520 rows of it 28.6 / 17.3); with 1.05, products of 1,600 rows and more lost 5 %.
+static bool tc_pairs(int M, int N, int K, bool gated, bool cut) {
+    if (M <= TC_BM) return false;
+    const int sms = tc_sm_count(), cols = gated ? TC_BN / 2 : TC_BN, tiles_n = (N + cols - 1) / cols;
+    const double pairs = tc_rounds((M + 2 * TC_BM - 1) / (2 * TC_BM) * tiles_n, sms / 2 > 0 ? sms / 2 : 1, K, cut);
+    const double single = tc_rounds((M + TC_BM - 1) / TC_BM * tiles_n, sms, K, cut);
+    return pairs <= 1.2 * single;
 }
 
 // A [M, K] and B [N, K] (or [2N, K] with epilogue 2) bfloat16 with row strides
@@ -747,7 +767,7 @@ TQ_API int tq_gemm_tc(const void* A, const void* B, const float* bias, void* C, 
     CUtensorMap ma, mb;
     int st = make_map(&ma, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, TC_BM);
     if (st) return st;
-    const bool pair = tc_mode() == 2 || (tc_mode() == 0 && M > TC_BM);
+    const bool pair = tc_mode() == 2 || (tc_mode() == 0 && tc_pairs(M, N, K, gated, epilogue == EPI_ACCUM));
     const uint64_t b_rows = gated ? 2ull * N : (uint64_t)N;
     // a block loads 128 rows of B at a time in the pair form and with SwiGLU, else the tile's 256
     st = make_map(&mb, B, b_rows, (uint64_t)K, (uint64_t)ldb, (pair || gated) ? TC_BN / 2 : TC_BN);
