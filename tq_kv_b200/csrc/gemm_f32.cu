@@ -1,5 +1,5 @@
-// The float32 products of many rows on float32 fused multiply-adds: C[M,N] (=, +=) A[M,K] · W[N,K]^T (+ bias[N]),
-// float32 operands and result, every sum in float32 (no tensor cores, no reduced-precision mode).  Optional epilogues:
+// Float32 products that gemm_f32_tc.cu does not take, on float32 fused multiply-adds:
+// C[M,N] (=, +=) A[M,K] · W[N,K]^T (+ bias[N]), float32 operands and result, every sum in float32 (no reduced-precision mode).  Optional epilogues:
 // W holding gate rows then up rows, C = act(gate) * up; or the square of relu.
 //
 // What bounds it: the 128 float32 lanes of an SM (about 72 TFLOP/s).  A block of 128 threads makes a tile of 64 x 128

@@ -112,7 +112,7 @@ class GQAttention(Mixer):
         packed = self._use_packed(b.host_start, b.host_lens, owns)
         # Where a decode step's q/k/v product adds shares of K into its result, the result must start at zero.
         # Instead of clearing it before every product, the layers share one buffer that is zero between uses:
-        # the rotary kernel, which alone reads it, leaves zeros behind.
+        # the rotary kernel (or the fused decode kernel), which alone reads it, leaves zeros behind.
         kept_zero = (T <= self.ZERO_BUFFER_ROWS and act == torch.bfloat16
                      and getattr(self.position, "clears_input", False)
                      and kernels.product_adds_shares(T, self.w_qkv, isinstance(x, kernels.PendingNorm)))
