@@ -195,11 +195,17 @@ latent_heads4_kernel(const float* __restrict__ q, int ldq, const float* __restri
     }
 }
 
+// blockIdx.z: `cols` of the head's e results.  Bound by the latency of reading U_v, so a warp reads four of its rows at a time, and
+// a head goes to several blocks while that fills the GPU; every sum is made in the same order however it is cut.  16 heads of 128 from
+// latents of 512, float32, U_v in the L2, a row at a time and a whole head a block / here, us: 1 token 28.6 / 5.0, 4 29.3 / 5.4, 64
+// 32.6 / 22.5, 74 33.9 / 31.2, 150 (whole heads here too) 69.2 / 57.6, 700 239 / 184.
+#define LE_COLS 16
 template <typename T>
-__global__ void latent_expand_kernel(const T* __restrict__ lat, int H, int n, int rp, int e, const T* __restrict__ uv,
-                                     const float* __restrict__ gate, int ldg, int head_gate, T* __restrict__ out) {
+__global__ void __launch_bounds__(128) latent_expand_kernel(const T* __restrict__ lat, int H, int n, int rp, int e, int cols,
+                                                            const T* __restrict__ uv, const float* __restrict__ gate, int ldg,
+                                                            int head_gate, T* __restrict__ out) {
     extern __shared__ float sh[];          // [n] the head's mean latent
-    const int t = blockIdx.x, h = blockIdx.y;
+    const int t = blockIdx.x, h = blockIdx.y, first = blockIdx.z * cols, end = min(e, first + cols);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     pdl_wait();
     pdl_launch();
@@ -207,7 +213,7 @@ __global__ void latent_expand_kernel(const T* __restrict__ lat, int H, int n, in
     for (int i = threadIdx.x; i < n; i += blockDim.x) sh[i] = to_f32<T>(lr[i]);
     __syncthreads();
     if (!uv) {                             // nothing to expand: the head's first e entries, gated
-        for (int j = threadIdx.x; j < e; j += blockDim.x) {
+        for (int j = first + threadIdx.x; j < end; j += blockDim.x) {
             const size_t c = (size_t)h * e + j;
             float acc = sh[j];
             if (gate) acc *= 1.f / (1.f + expf(-gate[(size_t)t * ldg + (head_gate ? h : c)]));
@@ -215,15 +221,24 @@ __global__ void latent_expand_kernel(const T* __restrict__ lat, int H, int n, in
         }
         return;
     }
-    for (int j = warp; j < e; j += n_warps) {
-        const T* w = uv + ((size_t)h * e + j) * n;
-        float acc = 0.f;
-        for (int i = lane; i < n; i += 32) acc = fmaf(to_f32<T>(w[i]), sh[i], acc);
-        acc = warp_sum(acc);
-        if (lane == 0) {
-            const size_t c = (size_t)h * e + j;
-            if (gate) acc *= 1.f / (1.f + expf(-gate[(size_t)t * ldg + (head_gate ? h : c)]));
-            out[(size_t)t * H * e + c] = from_f32<T>(acc);
+    for (int j = first + warp * 4; j < end; j += n_warps * 4) {
+        const T* w[4];
+        float acc[4] = {};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) w[u] = uv + ((size_t)h * e + min(j + u, end - 1)) * n;
+#pragma unroll 4
+        for (int i = lane; i < n; i += 32) {
+            const float x = sh[i];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc[u] = fmaf(to_f32<T>(w[u][i]), x, acc[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] = warp_sum(acc[u]);
+        if (lane < 4 && j + lane < end) {
+            float v = lane == 0 ? acc[0] : lane == 1 ? acc[1] : lane == 2 ? acc[2] : acc[3];
+            const size_t c = (size_t)h * e + j + lane;
+            if (gate) v *= 1.f / (1.f + expf(-gate[(size_t)t * ldg + (head_gate ? h : c)]));
+            out[(size_t)t * H * e + c] = from_f32<T>(v);
         }
     }
 }
@@ -438,13 +453,16 @@ TQ_API int tq_latent_expand(const void* lat, int H, int n, int rp, int e, const 
                              LpQuery{0, 0, 0, 0, 0, nullptr, nullptr, nullptr}, gate, ldg, head_gate,
                              (int)(!((rp | n) & 3) && (reinterpret_cast<uintptr_t>(lat) & 7) == 0));
     const size_t smem = (size_t)n * sizeof(float);
-    const dim3 grid(n_tokens, H);
+    // a head in pieces of 16 results while whole heads give an SM fewer than eight blocks
+    int cols = e;
+    if (uv && (long long)n_tokens * H < 8ll * tq_sm_count() && (e + LE_COLS - 1) / LE_COLS <= 65535) cols = LE_COLS;
+    const dim3 grid(n_tokens, H, (e + cols - 1) / cols);
     if (dtype == TQ_F32)
         return tq_launch_pdl(TQ_PDL_ELEMENTWISE, latent_expand_kernel<float>, grid, dim3(128), smem, stream,
-                             (const float*)lat, H, n, rp, e, (const float*)uv, gate, ldg, head_gate, (float*)out);
+                             (const float*)lat, H, n, rp, e, cols, (const float*)uv, gate, ldg, head_gate, (float*)out);
     if (dtype == TQ_BF16)
         return tq_launch_pdl(TQ_PDL_ELEMENTWISE, latent_expand_kernel<bf16>, grid, dim3(128), smem, stream,
-                             (const bf16*)lat, H, n, rp, e, (const bf16*)uv, gate, ldg, head_gate, (bf16*)out);
+                             (const bf16*)lat, H, n, rp, e, cols, (const bf16*)uv, gate, ldg, head_gate, (bf16*)out);
     return (int)cudaErrorInvalidValue;
 }
 
